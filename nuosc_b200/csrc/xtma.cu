@@ -1,35 +1,52 @@
 // xtma.cu -- TMA-fed x-march stage kernel (the fast path of the fused stage).
 //
-// Same arithmetic and per-thread structure as xmarch.cu (one (z, v) column per
-// thread -- two adjacent velocities per thread in FP32 --, a (2R+1)-deep
-// register queue in x, fused RK epilogue and moment partials), with
-// Blackwell-native data movement:
-//   * box ring: for every x plane the CTA touches, lane 0 of warp 0 issues one
-//     TMA tensor load (cp.async.bulk.tensor.4d; 2-3 boxes where the periodic z
-//     wrap cuts it) of the plane's [TZ+2R rows][4 fields][VB velocities] box
-//     and a bulk copy of the TZ cells' moments into a ring slot whose
-//     completion is tracked by a "full" mbarrier (expect_tx bytes).  A box is
-//     used twice: first as the queue front (x+R), R planes later as the
-//     centre plane of the z stencil, so each state value crosses HBM once;
-//   * warps never exchange data and there is no CTA-wide barrier in the
-//     march: a warp waits only on full barriers and releases a slot after its
-//     last use by arriving on the slot's "empty" mbarrier; the issuing lane
-//     waits on "empty" before refilling a slot;
-//   * the pointwise inputs of the epilogue (U in S2 and S3, U and B in S4;
-//     none in S1) are plain coalesced loads issued at the top of each plane,
-//     before the waits and the stencil; the issuing lane prefetches their TZ
-//     rows into L2 two planes ahead with a tensor prefetch
-//     (cp.async.bulk.prefetch.tensor), so the loads find them in L2;
+// A CTA owns TZ z rows x one velocity block (32 velocities in FP64, 64 in FP32)
+// x one flavour half and marches along x:
+//   * a producer warpgroup (one issuing lane) loads, for every x plane the CTA
+//     touches, the plane's [TZ+2R rows][4 fields][velocities] box with one TMA
+//     tensor load (cp.async.bulk.tensor.4d; 2-3 boxes where the periodic z wrap
+//     cuts it), the TZ cells' moments with a bulk copy, and the stage's
+//     pointwise input (U in S2 and S3, B in S4; none in S1) of the plane that
+//     the box completes, into shared-memory rings whose completion is tracked
+//     by "full" mbarriers (expect_tx bytes).  A box is used twice: as the front
+//     (x+R) of the march, where all its rows enter the stencil sums, and R
+//     planes later for its centre values, so each state value crosses HBM once;
+//   * consumer warps never exchange data and there is no CTA-wide barrier in
+//     the march: a warp waits only on full barriers and arrives on a slot's
+//     "empty" barrier after its last use;
+//   * each consumer thread owns two z rows of one 8-byte value (a double, or two
+//     floats in packed arithmetic) per field: the 2R+2 rows it reads from a box
+//     serve both rows' z stencils (8 shared loads per field for two points
+//     instead of 14), and the per-velocity constants are held in registers;
+//   * the x stencil is kept in transposed form: 2R partial sums per value,
+//     each front value added to all of them, so nothing is shifted and the
+//     products of a value do not depend on each other;
 //   * moment partials (FP64 products and sums; FP32 state may sum in float
-//     within the block, stored as double): each lane forms its 12 products
-//     (3 combinations x 4 weights, the weights in a lane-permuted order set
-//     once per tile) and the warp reduce-scatters them over its 32 lanes
-//     with 13 shuffle-adds;
+//     within the block, stored as double): a warp's half-warps exchange values
+//     so that each keeps one row, each lane forms the 12 products (3
+//     combinations x 4 weights, the weights in a lane-permuted order set once
+//     per tile) of its own and its partner's velocities, and the half-warp
+//     reduce-scatters them with 12 shuffle-adds;
 //   * a stopped instance of a batch (its halt flag set by the device-side
 //     stop test) has its tiles skipped.
 // All mbarrier waits are bounded: on expiry the kernel records the timeout in
 // the status word, stops marching and, before returning, waits (again
 // bounded) for the copies it issued.  Requires nz % TZ == 0.
+//
+// What bounds it, measured on a 512 x 256 x 642 FP64 grid (KO6): S1 2.8 ms (2
+// state passes, 3.9 TB/s) is held by instruction latency at 8 consumer warps
+// per SM (two per scheduler: the partial sums alone take 96 registers); S2 4.5,
+// S3 3.1, S4 3.2 ms run at 4.8-5.2 TB/s of the 6.5 a plain copy reaches.  The
+// form before -- 16 warps of one point per thread, a 7-deep register queue in x
+// shifted every plane, weights read from shared memory, plain loads of the
+// pointwise inputs, warp 0 issuing the copies -- took 3.9 / 5.0 / 4.5 / 4.6 ms:
+// 404-467 instructions and 112 shared-memory wavefronts per 32 points against
+// 225-260 and 70 now, with the shared-memory pipe at 65 %.  Tried between the
+// two, on the same grid (S1): two velocities per thread 3.8 (constants re-read
+// from shared memory: its pipe stays the limit), the fields split between
+// warps 4.0 (same), the issue rotated among the consumer warps 2.9 but S2 6.2
+// (a late warp starves all), issue by the last warp to release a slot 3.3.
+// FP32 (same grid): 2.2 / 2.8 / 2.4 / 2.5 -> 1.7 / 2.2 / 1.8 / 1.8 ms.
 //
 // The march of one tile is a device function shared by two kernels: k_xtma
 // (one tile per CTA, one instance per launch) and k_xtma_batch (a persistent
@@ -41,6 +58,7 @@
 
 #include <cstring>
 #include <type_traits>
+#include <utility>
 
 namespace nuosc {
 
@@ -51,23 +69,88 @@ namespace {
 // polls give up after about 1 s
 constexpr unsigned kWaitSpins = 1u << 18;
 
-// velocities per thread and per CTA: FP32 threads take two adjacent velocities
+// One 8-byte value of the march: a double, or two floats of adjacent velocities
+// in one register pair (packed f32x2 arithmetic).  A thread owns one such value
+// per row and field, so a warp covers 32 velocities in FP64 and 64 in FP32, and
+// RW z rows.  Every product that is added to something is an explicit fma and
+// the other operations are not contracted, so all kernels that share the march
+// round alike (a batch member equals its solo run bit for bit).
 template <typename T>
 constexpr int vpt() {
-    return sizeof(T) == 4 ? 2 : 1;
+    return 8 / (int)sizeof(T);
 }
 template <typename T>
 constexpr int vblock() {
     return 32 * vpt<T>();
 }
+constexpr int RW = 2;
+constexpr int threads_of(int tz) { return 32 * (tz / RW) + 128; }  // consumer warps and the producer's warpgroup
+
+struct f2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f2 pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double vmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double vsub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double vneg(double a) { return -a; }
+__device__ __forceinline__ f2 vfma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f2 vadd(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 vmul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 vsub(f2 a, f2 b) { return vfma(b, pack(-1.f, -1.f), a); }
+__device__ __forceinline__ f2 vneg(f2 a) { return f2{a.v ^ 0x8000000080000000ull}; }
+
+template <typename T>
+struct VecOf;
+template <>
+struct VecOf<double> {
+    using V = double;
+    static __device__ __forceinline__ V splat(double x) { return x; }
+    static __device__ __forceinline__ V make(const double (&x)[1]) { return x[0]; }
+    static __device__ __forceinline__ void get(V a, double (&x)[1]) { x[0] = a; }
+    static __device__ __forceinline__ V ld(const double *p) { return *p; }
+    static __device__ __forceinline__ void st(double *p, V a) { *p = a; }
+    static __device__ __forceinline__ V zero() { return 0.0; }
+};
+template <>
+struct VecOf<float> {
+    using V = f2;
+    static __device__ __forceinline__ V splat(double x) { return pack((float)x, (float)x); }
+    static __device__ __forceinline__ V make(const double (&x)[2]) { return pack((float)x[0], (float)x[1]); }
+    static __device__ __forceinline__ void get(V a, float (&x)[2]) {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(a.v));
+    }
+    static __device__ __forceinline__ V ld(const float *p) {
+        return f2{*reinterpret_cast<const unsigned long long *>(p)};
+    }
+    static __device__ __forceinline__ void st(float *p, V a) { *reinterpret_cast<unsigned long long *>(p) = a.v; }
+    static __device__ __forceinline__ V zero() { return f2{0ull}; }
+};
 
 struct __align__(64) TmaMaps {
     CUtensorMap zr;   // box of TZ+2R rows (plane box with both halos)
     CUtensorMap tzr;  // TZ+R rows (a box cut by the wrap)
     CUtensorMap tz;   // TZ rows (middle piece of a box wrapped at both ends)
     CUtensorMap r;    // R rows (wrapped halo)
-    CUtensorMap pu;   // TZ rows of the stage's U register (L2 prefetch of the pointwise input)
-    CUtensorMap pa;   // TZ rows of the final stage's B input (acc_src; L2 prefetch)
+    CUtensorMap pu;   // TZ rows of the stage's U register (pointwise input)
+    CUtensorMap pa;   // TZ rows of the final stage's B input (acc_src; pointwise)
     // the same four box shapes over a slab's halo buffer (planes right of the slab)
     CUtensorMap hzr, htzr, htz, hr;
 };
@@ -82,6 +165,15 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
 }
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// register split between the warpgroups of a CTA (RegSplit)
+template <int N>
+__device__ __forceinline__ void setmaxnreg_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void setmaxnreg_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(N));
 }
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigned spins = kWaitSpins) {
     for (unsigned it = 0; it < spins; ++it) {
@@ -110,34 +202,10 @@ __device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap *map
         "l"((unsigned long long)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
         : "memory");
 }
-// L2 prefetch of one tensor box: no shared memory, no completion to wait for
-__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap *map, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
-                     (unsigned long long)map),
-                 "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
-}
 __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
-}
-
-// VPT consecutive values (8-byte vector access when VPT == 2)
-template <typename T, int N>
-__device__ __forceinline__ void ldv(const T *p, T (&o)[N]) {
-    if constexpr (N == 2) {
-        const float2 t = *reinterpret_cast<const float2 *>(p);
-        o[0] = t.x;
-        o[1] = t.y;
-    } else {
-        o[0] = *p;
-    }
-}
-template <typename T, int N>
-__device__ __forceinline__ void stv(T *p, const T (&o)[N]) {
-    if constexpr (N == 2) *reinterpret_cast<float2 *>(p) = make_float2(o[0], o[1]);
-    else *p = o[0];
 }
 
 constexpr int up128(int x) { return (x + 127) / 128 * 128; }
@@ -161,94 +229,45 @@ struct Slot {
 //         difference before its factor f = -v/(12 dx)),
 // is evaluated as one weighted sum per axis: the four neighbours at offsets
 // -2, -1, +1, +2 carry per-velocity weights (KO and ADV coefficients folded
-// together, StencilW), the pair at +-3 (6th difference only) the uniform
+// together, stencil_weights), the pair at +-3 (6th difference only) the uniform
 // eps, and the centre, shared by both axes, -20 (eps_z + eps_x) or
 // 6 (eps_z + eps_x).  That is 14 (6th) or 10 (4th) FP64 operations per field
 // instead of 22 (18) for the separate KO and ADV sums.
 //   6th: w = {-6 eps + f, 15 eps - 8 f, 15 eps + 8 f, -6 eps - f}
 //   4th: w = {eps + f, -4 eps - 8 f, -4 eps + 8 f, eps - f}
 template <int R>
-__host__ __device__ __forceinline__ void stencil_weights(double eps, double f, double (&w)[4]) {
+__device__ __forceinline__ void stencil_weights(double eps, double f, double (&w)[4]) {
     if (R == 3) {
-        w[0] = -6 * eps + f;
-        w[1] = 15 * eps - 8 * f;
-        w[2] = 15 * eps + 8 * f;
-        w[3] = -6 * eps - f;
+        w[0] = fma(-6.0, eps, f);
+        w[1] = fma(15.0, eps, -8 * f);
+        w[2] = fma(15.0, eps, 8 * f);
+        w[3] = fma(-6.0, eps, -f);
     } else {
-        w[0] = eps + f;
-        w[1] = -4 * eps - 8 * f;
-        w[2] = -4 * eps + 8 * f;
-        w[3] = eps - f;
+        w[0] = __dadd_rn(eps, f);
+        w[1] = fma(-4.0, eps, -8 * f);
+        w[2] = fma(-4.0, eps, 8 * f);
+        w[3] = __dsub_rn(eps, f);
     }
 }
 
-// one axis's off-centre terms: s[C-2..C+2] without the centre with weights
-// w[0..3], plus eps (s[0] + s[6]) in the 6th difference
-template <typename T, int R>
-__device__ __forceinline__ T axis_sum(const T (&s)[2 * R + 1], const T (&w)[4], T eps) {
-    constexpr int C = R;
-    T acc;
-    if constexpr (R == 3) acc = eps * (s[0] + s[6]);
-    else acc = T(0);
-    acc = fma(w[0], s[C - 2], acc);
-    acc = fma(w[1], s[C - 1], acc);
-    acc = fma(w[2], s[C + 1], acc);
-    return fma(w[3], s[C + 2], acc);
+// inp (physics.cuh) with its fmas explicit
+__device__ __forceinline__ double contract4(const double *m, double vx, double vy, double vz) {
+    return fma(-m[3], vz, fma(-m[2], vy, fma(-m[1], vx, m[0])));
 }
 
-template <typename T, bool VAC>
-__device__ __forceinline__ void rhs_half(const T (&c)[4], T a, T b, T e, T mu, T p2s, T p2c, T ps, const T (&sten)[4],
-                                         T (&out)[4], bool vac) {
-    const T ee = c[0], mm = c[1], emr = c[2], emi = c[3];
-    const T Iee = T(2) * mu * (emi * a + emr * b);
-    const T Iemr = -mu * ((ee - mm) * b + e * emi);
-    const T Iemi = mu * ((mm - ee) * a + e * emr);
-    out[0] = Iee + sten[0];
-    out[1] = -Iee + sten[1];
-    out[2] = Iemr + sten[2];
-    out[3] = Iemi + sten[3];
-    if (VAC && vac) {  // pmo * [H_vac, rho] (nuosc_class.cpp:280-287); p2s = 2 pmo st, p2c = 2 pmo ct, ps = pmo st
-        out[0] -= p2s * emi;
-        out[1] += p2s * emi;
-        out[2] -= p2c * emi;
-        out[3] += p2c * emr + ps * (ee - mm);
-    }
+// s/3 + t as third_plus (physics.cuh)
+template <typename T>
+__device__ __forceinline__ typename VecOf<T>::V vthird_plus(typename VecOf<T>::V s, typename VecOf<T>::V t) {
+    using O = VecOf<T>;
+    const auto third = O::splat(1.0 / 3.0);
+    const auto q = vmul(s, third);
+    const auto r = vfma(q, O::splat(-3.0), s);
+    return vadd(q, vfma(r, third, t));
 }
 
-// the weights 2jj and 2jj + 1 of this lane's NP velocities (one 16-byte load)
-template <typename T, int NP>
-__device__ __forceinline__ void ldw(const T *p, T (&a)[NP], T (&b)[NP]) {
-    if constexpr (NP == 2) {
-        const float4 t = *reinterpret_cast<const float4 *>(p);
-        a[0] = t.x;
-        a[1] = t.y;
-        b[0] = t.z;
-        b[1] = t.w;
-    } else {
-        const double2 t = *reinterpret_cast<const double2 *>(p);
-        a[0] = t.x;
-        b[0] = t.y;
-    }
-}
-
-// statically allocated per-CTA scratch of the march: the abort flag, the
-// per-velocity stencil weights and, with two velocities per thread (FP32),
-// the per-velocity constants of the commutator and the moments (the moment
-// weights in double when the FP32 march sums its moment partials in FP64, M64)
-template <typename T, bool M64>
+// statically allocated per-CTA scratch of the march
 struct MarchShared {
-    static constexpr bool kShared = vpt<T>() == 2;
-    static constexpr int NP = vpt<T>();
-    // [component][lane] and [j][lane], the lane's two velocities side by side
-    // (one 16-byte load, 8-byte for float weights); consecutive lanes read
-    // consecutive vectors (a lane-major layout would put 16 lanes on one bank)
-    double2 vq[kShared ? 3 : 1][kShared ? 32 : 1];                              // vx, vy, vz
-    std::conditional_t<M64, double2, float2> wp[kShared ? 4 : 1][kShared ? 32 : 1];  // lane-permuted
-    // stencil weights, z axis j = 0..3 then x axis j = 4..7, in pairs: sw[jj][lane]
-    // holds weights 2jj (NP velocities) and 2jj + 1 (NP velocities), 16 bytes,
-    // so a lane reads all eight with four conflict-free 16-byte loads
-    __align__(16) T sw[4][32][2 * NP];
-    int abort;
+    int abort;  // a bounded wait expired
 };
 
 template <typename T, int TZ>
@@ -256,23 +275,31 @@ constexpr int tma_ctas_per_sm() {
     return TZ == 16 ? 1 : 2;
 }
 
-// Ring geometry of one march.  Boxes are issued D planes ahead of their
-// front use: 3 with 16-row tiles (one CTA per SM, 8 slots of 24 KB at R = 3),
-// 2 with 8-row tiles (two CTAs per SM share the 228 KB).  The pointwise
-// inputs of the epilogue (U in S2/S3/S4, B in S4) stay plain
-// per-thread loads, but thread 0 prefetches their TZ rows of plane x + PFD
-// into L2 with one tensor prefetch each, so those loads hit L2: measured 3 %
-// faster per step than without (PFD 1 and 3 equal within noise, 6 slower),
-// and faster than staging them through shared memory, which costs ring depth.
+// Ring geometry of one march.  A box lives from its issue, D planes ahead of
+// its front use, to its centre use, R planes after it; a stage with a pointwise
+// input (U in S2 and S3, B in S4) has a second ring of D plane pieces of it.  D
+// is what the shared memory of one (TZ = 16) or two (TZ = 8) CTAs per SM holds.
 template <typename T, int R, int MODE, int TZ>
 struct MarchCfg {
-    static constexpr int D = TZ == 16 ? 3 : 2;  // boxes issued ahead of their first use
-    static constexpr int PFD = 2;                 // L2 prefetch distance of the pointwise inputs, planes
     static constexpr bool PU = MODE == MODE_SY || MODE == MODE_S2B;  // reads U pointwise
     static constexpr bool PA = MODE == MODE_S4B;                     // reads B pointwise
-    static constexpr int NS = R + D + 2;  // a box lives from its front use to its centre use, plus slack
+    static constexpr bool PW = PU || PA;
+    static constexpr int D = PW ? (R == 3 ? 3 : 4) : (TZ == 8 && R == 3 ? 4 : 5);
+    static constexpr int NS = R + D;
+    static constexpr int PS = PW ? D : 0, PSM = PW ? D : 1;
+    static constexpr unsigned pbytes = sizeof(T) * TZ * 4 * vblock<T>();
     static constexpr size_t ring = (size_t)NS * Slot<T, TZ, R>::bytes;
-    static constexpr size_t smem = ring + 2 * NS * 8;  // box ring | mbarriers
+    static constexpr size_t bars = ring + PS * pbytes;
+    static constexpr size_t smem = bars + 2 * NS * 8;  // box ring | pointwise ring | mbarriers
+};
+
+// Registers per thread after the split: a CTA starts with the even share of the
+// SM's 65,536 (168 for 256 + 128 threads, 128 for two CTAs of 128 + 128), its
+// producer warpgroup gives up all but `producer`, which is what the consumers
+// take: 256 x 232 + 128 x 40 = 384 x 168, 128 x 216 + 128 x 40 = 256 x 128.
+template <int TZ>
+struct RegSplit {
+    static constexpr int producer = 40, consumer = TZ == 16 ? 232 : 216;
 };
 
 }  // namespace
@@ -286,35 +313,125 @@ __device__ __forceinline__ P rd(const P &x) {
 }
 
 // One tile of work: z rows z0..z0+TZ-1, velocity block vb (of nvb), x planes
-// xs..xe-1, flavour half `half`, of the instance described by (*mp, a).
-// Called by the single-instance kernel (one tile per CTA; a and *mp in kernel
-// parameter space) and by the persistent batched kernel (many tiles per CTA,
-// of many instances; SA: a and mp in shared memory); the arithmetic per
-// (cell, velocity) does not depend on which.  VAC compiles the vacuum term in
-// (it then runs where a.c.pmo != 0).  Returns true when a bounded wait
-// expired (the status word is set and the tile is incomplete).
-template <typename T, int R, int MODE, int TZ, bool VAC, bool SA, bool M64>
-__device__ __forceinline__ bool xtma_march(const TmaMaps *const &mp, const StageArgs<T> &a, const int z0, const int vb,
-                                           const int nvb, const int xs, const int xe, const int half,
-                                           unsigned char *smem, MarchShared<T, M64> &sh) {
+// xs..xe-1, flavour half `half`
+struct Tile {
+    int z0, vb, nvb, xs, xe, half;
+};
+
+// The march of one tile of the instance (maps, a): every thread of the CTA calls
+// xtma_produce (the last warpgroup) or xtma_consume (the others); both return
+// true when a bounded wait expired (the status word is set and the tile is
+// incomplete).  Called by the single-instance kernel (one tile per CTA; a and
+// maps in kernel parameter space) and by the persistent batched kernel (many
+// tiles per CTA, of many instances; SA: a in shared memory); the arithmetic per
+// (cell, velocity) does not depend on which.
+//
+// Producer: one lane loads box j (plane xs + j, periodic) and, for the stages
+// with a pointwise input, that input's TZ rows of plane j - R, into slots
+// j % NS and (j - R) % PS; one full barrier per box slot (phase j / NS) counts
+// the bytes of both.  It may refill a slot when every consumer warp has
+// arrived on the slot's empty barrier, D planes later.
+// fault_tx (the self-test of the bounded waits) over-declares the bytes of box
+// R of the instance's first tile: all its copies land, its phase never completes.
+template <typename T, int R, int MODE, int TZ, bool M64>
+__device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArgs<T> &a, const Tile &t,
+                                             unsigned char *smem, MarchShared &sh) {
     using S = Slot<T, TZ, R>;
     using CF = MarchCfg<T, R, MODE, TZ>;
-    constexpr int NP = vpt<T>();       // velocities per thread
-    constexpr int VB = S::VB;          // velocities per CTA
-    constexpr int W = 2 * R + 1;
-    constexpr int ZR = S::ZR;
-    constexpr int D = CF::D;
+    constexpr int NS = CF::NS, ZR = S::ZR;
+    unsigned long long *bars = (unsigned long long *)(smem + CF::bars);  // full[NS], empty[NS]
+    const bool lead = threadIdx.x == 32 * (TZ / RW);
+    if (lead) {
+        sh.abort = 0;
+        for (int s = 0; s < 2 * NS; ++s) mbar_init(smem_u32(&bars[s]), s < NS ? 1u : (unsigned)(TZ / RW));
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    int issued = 0;  // last box issued + 1
+    if (lead) {
+        const int nx = a.g.nx, nz = a.g.nz, c0 = t.vb * S::VB, c1 = 4 * t.half, nplanes = t.xe - t.xs;
+        const bool halo = a.halo != nullptr;
+        for (int j = 0; j < nplanes + R; ++j) {  // centres xs..xe-1 and fronts up to xe-1+R
+            const int s = j % NS;
+            if (j >= NS && (*(volatile int *)&sh.abort ||
+                            !mbar_wait(smem_u32(&bars[NS + s]), (unsigned)((j / NS - 1) & 1)))) {
+                sh.abort = 1;
+                break;
+            }
+            const unsigned full = smem_u32(&bars[s]);
+            unsigned char *sp = smem + s * S::bytes;
+            const bool pw = CF::PS > 0 && j >= R;
+            unsigned tx = S::tx + (pw ? CF::pbytes : 0u);
+            if (j == R && t.z0 == 0 && t.vb == 0 && t.xs == 0 && t.half == 0) tx += a.fault_tx;
+            mbar_expect_tx(full, tx);
+            // past the last plane it wraps (periodic) or, in a slab, comes from
+            // the halo buffer's right planes (box plane x - nx + R).  Boxes
+            // start at plane xs >= 0, so the left halo is never a box.
+            const int xl = t.xs + j;  // < nx + R < 2 nx
+            const bool hal = xl >= nx && halo;
+            const int x = hal ? xl - nx + R : xl >= nx ? xl - nx : xl;
+            // 1 piece, or 2-3 where the periodic z wrap cuts the box
+            int zstart = t.z0 - R, dst = 0;
+            while (dst < ZR) {
+                const int zw = zstart < 0 ? zstart + nz : (zstart >= nz ? zstart - nz : zstart);
+                int len = nz - zw;
+                if (len > ZR - dst) len = ZR - dst;
+                const CUtensorMap *m = len == ZR        ? (hal ? &maps.hzr : &maps.zr)
+                                       : len == TZ + R ? (hal ? &maps.htzr : &maps.tzr)
+                                       : len == TZ     ? (hal ? &maps.htz : &maps.tz)
+                                                       : (hal ? &maps.hr : &maps.r);
+                tma_load_4d(smem_u32(sp + S::box + dst * 4 * S::VB * sizeof(T)), m, c0, c1, zw, x, full);
+                zstart += len;
+                dst += len;
+            }
+            // the cell moments are read at a box's centre use, which is always an
+            // interior plane; a halo box (front use only) loads plane nx-1's, unread
+            const int xm = hal ? nx - 1 : x;
+            bulk_load(smem_u32(sp + S::mb), a.mom_in + ((long long)xm * nz + t.z0) * NMOM, 8u * TZ * NMOM, full);
+            if (pw)
+                tma_load_4d(smem_u32(smem + CF::ring + (j - R) % CF::PSM * CF::pbytes), CF::PU ? &maps.pu : &maps.pa, c0,
+                            c1, t.z0, t.xs + j - R, full);
+            issued = j + 1;
+        }
+    }
+    __syncthreads();
+    const bool aborted = sh.abort != 0;
+    if (lead) {
+        if (aborted) {
+            // a wait expired: report it, then wait (bounded) for the copies of
+            // the last NS boxes issued -- the only ones that may still be in
+            // flight: box j - NS of a slot was consumed (so had landed) before
+            // box j was issued into it -- before the CTA's shared memory is
+            // reused or released
+            atomicExch(a.status, NUOSC_TIMEOUT_CODE);
+            for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
+                mbar_wait(smem_u32(&bars[j % NS]), (unsigned)((j / NS) & 1));
+        }
+        for (int s = 0; s < 2 * NS; ++s) mbar_inval(smem_u32(&bars[s]));
+    }
+    return aborted;
+}
+
+// VAC compiles the vacuum term in (it then runs where a.c.pmo != 0).
+template <typename T, int R, int MODE, int TZ, bool VAC, bool SA, bool M64>
+__device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &t, unsigned char *smem,
+                                             MarchShared &sh) {
+    using S = Slot<T, TZ, R>;
+    using CF = MarchCfg<T, R, MODE, TZ>;
+    using O = VecOf<T>;
+    using V = typename O::V;
+    constexpr int NP = vpt<T>();  // velocities per thread
+    constexpr int VB = S::VB;     // velocities per CTA
     constexpr int NS = CF::NS;
-    unsigned long long *bars = (unsigned long long *)(smem + CF::ring);  // full[NS], empty[NS]
-    int &s_abort = sh.abort;
+    unsigned long long *bars = (unsigned long long *)(smem + CF::bars);  // full[NS], empty[NS]
 
     const Geom g = a.g;
-    const int tid = threadIdx.x, lane = tid & 31, r = tid >> 5;
+    const int z0 = t.z0, vb = t.vb, nvb = t.nvb, xs = t.xs, half = t.half;
+    const int lane = threadIdx.x & 31, r = (threadIdx.x >> 5) * RW;  // this warp's rows r, r + 1
     const int v = vb * VB + NP * lane;  // first of this thread's NP velocities
     const bool vact = v < g.nvs;        // nvs is a multiple of NP, so all NP are active together
-    const int nplanes = xe - xs;
-    const int nboxes = nplanes + R;    // centres xs..xe-1 and fronts up to xe-1+R
-    const int zr = z0 + r;             // < nz since nz % TZ == 0
+    const int nplanes = t.xe - xs, nboxes = nplanes + R;
+    const int zr = z0 + r;  // < nz since nz % TZ == 0
     const long long fs = g.fs;
     const long long P = (long long)g.nz * g.nvs;
     const long long hoff = (long long)half * 4 * fs;
@@ -326,386 +443,297 @@ __device__ __forceinline__ bool xtma_march(const TmaMaps *const &mp, const Stage
     // all fit (xtma_supported requires 3 fs < 2^32); only the half's own
     // offset, hoff, needs 64 bits
     const unsigned fs32 = (unsigned)fs, P32 = (unsigned)P, own32 = (unsigned)own;
+    __syncthreads();  // the barriers are initialised
 
-    __syncthreads();  // the previous tile of this CTA (batched kernel) is done with the ring
-    if (tid == 0) {
-        s_abort = 0;
-        for (int s = 0; s < 2 * NS; ++s) mbar_init(smem_u32(&bars[s]), s < NS ? 1u : (unsigned)TZ);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    __syncthreads();
-
-    // lane 0 of warp 0: load box j (plane xs + j, periodic) into slot j % NS
-    // (phase j / NS of its full barrier).  `issued` = last box issued + 1.
-    // fault_tx (the self-test of the bounded waits) over-declares the bytes of
-    // box R of the instance's first tile: all its copies land, its phase never
-    // completes.
-    int issued = 0;
-    const unsigned fault_tx =
-        (tid == 0 && z0 == 0 && vb == 0 && xs == 0 && half == 0) ? rd<SA>(a.fault_tx) : 0u;
-    auto issue = [&](int j) -> bool {
-        const int s = j % NS;
-        if (j >= NS && !mbar_wait(smem_u32(&bars[NS + s]), (unsigned)((j / NS - 1) & 1))) return false;
-        const unsigned full = smem_u32(&bars[s]);
-        unsigned char *sp = smem + s * S::bytes;
-        mbar_expect_tx(full, S::tx + (j == R ? fault_tx : 0u));
-        // plane xs + j; past the last plane it wraps (periodic) or, in a slab,
-        // comes from the halo buffer's right planes (box plane x - nx + R).
-        // Boxes start at plane xs >= 0, so the left halo is never a box.
-        const int nx = rd<SA>(a.g.nx), xl = xs + j;
-        const bool hal = xl >= nx && rd<SA>(a.halo) != nullptr;
-        const int x = hal ? xl - nx + R : xl % nx;
-        const int nz = rd<SA>(a.g.nz);
-        const TmaMaps &maps = *rd<SA>(mp);
-        const int c1 = 4 * half, c0 = vb * VB;
-        int zstart = z0 - R, dst = 0;
-        while (dst < ZR) {
-            const int zw = zstart < 0 ? zstart + nz : (zstart >= nz ? zstart - nz : zstart);
-            int len = nz - zw;
-            if (len > ZR - dst) len = ZR - dst;
-            const CUtensorMap *m = len == ZR        ? (hal ? &maps.hzr : &maps.zr)
-                                   : len == TZ + R ? (hal ? &maps.htzr : &maps.tzr)
-                                   : len == TZ     ? (hal ? &maps.htz : &maps.tz)
-                                                   : (hal ? &maps.hr : &maps.r);
-            tma_load_4d(smem_u32(sp + S::box + dst * 4 * VB * sizeof(T)), m, c0, c1, zw, x, full);
-            zstart += len;
-            dst += len;
-        }
-        // the cell moments are read at a box's centre use, which is always an
-        // interior plane; a halo box (front use only) loads plane nx-1's, unread
-        const int xm = hal ? nx - 1 : x;
-        bulk_load(smem_u32(sp + S::mb), rd<SA>(a.mom_in) + ((long long)xm * nz + z0) * NMOM, 8u * TZ * NMOM, full);
-        issued = j + 1;
-        return true;
-    };
-
-    // thread 0: L2 prefetch of the pointwise inputs of plane xs + i
-    auto l2pref = [&](int i) {
-        if ((CF::PU || CF::PA) && i < nplanes) {
-            const TmaMaps &maps = *rd<SA>(mp);
-            if (CF::PU) tma_prefetch_4d(&maps.pu, vb * VB, 4 * half, z0, xs + i);
-            if (CF::PA) tma_prefetch_4d(&maps.pa, vb * VB, 4 * half, z0, xs + i);
-        }
-    };
-
-    // per-velocity and uniform constants.  Lane-permuted moment weights: slot s
-    // of this lane holds weight s ^ wq (weights w, w vx, w vy, w vz), wq = lane
-    // bits 4..3, the order the moment reduce-scatter needs.  With two
-    // velocities per thread (FP32) the per-velocity constants (FP64
-    // velocities, float weights) live in shared memory and are read per plane,
-    // which keeps the register queue clear of spills.
-    const int wq = (lane >> 3) & 3;
-    constexpr bool kShared = MarchShared<T, M64>::kShared;
-    auto &s_vq = sh.vq;
-    auto &s_wp = sh.wp;
-    double vxd[NP], vyd[NP], vzd[NP], wperm[NP][4];
+    // per-velocity constants, in registers.  Lane-permuted moment weights: slot s
+    // of a lane holds weight s ^ wq (weights w, w vx, w vy, w vz), wq = lane bits
+    // 3..2, the order the moment reduce-scatter needs; of this lane's
+    // velocities and of its partner's (lane ^ 16).
+    using M = std::conditional_t<M64, double, float>;
+    const int wq = (lane >> 2) & 3;
+    const int vp = vb * VB + NP * (lane ^ 16);
+    double vx[NP], vy[NP], vz[NP];
+    M wo[NP][4], wp[NP][4];
+    V wz[4], wx[4];
+    {
+        double tz[4][NP], tx[4][NP];
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        vxd[p] = a.q.vx[vc + p];
-        vyd[p] = a.q.vy[vc + p];
-        vzd[p] = a.q.vz[vc + p];
-        if (r == 0) {
-            double wz[4], wx[4];
-            stencil_weights<R>(a.c.kz, vzd[p] * a.c.fzs, wz);
-            stencil_weights<R>(a.c.kx, vxd[p] * a.c.fxs, wx);
+        for (int p = 0; p < NP; ++p) {
+            vx[p] = a.q.vx[vc + p];
+            vy[p] = a.q.vy[vc + p];
+            vz[p] = a.q.vz[vc + p];
+            double w4z[4], w4x[4];
+            stencil_weights<R>(a.c.kz, __dmul_rn(vz[p], a.c.fzs), w4z);
+            stencil_weights<R>(a.c.kx, __dmul_rn(vx[p], a.c.fxs), w4x);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                sh.sw[j >> 1][lane][(j & 1) * NP + p] = T(wz[j]);
-                sh.sw[2 + (j >> 1)][lane][(j & 1) * NP + p] = T(wx[j]);
-            }
-        }
-        const double wd = vact ? a.q.vw[vc + p] : 0.0;
-        const double v4w[4] = {wd, vxd[p] * wd, vyd[p] * wd, vzd[p] * wd};
+            for (int j = 0; j < 4; ++j) tz[j][p] = w4z[j], tx[j][p] = w4x[j];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int k = j ^ wq;
-            wperm[p][j] = k == 0 ? v4w[0] : k == 1 ? v4w[1] : k == 2 ? v4w[2] : v4w[3];
-        }
-    }
-    if constexpr (kShared) {
-        if (r == 0) {
-            s_vq[0][lane] = make_double2(vxd[0], vxd[NP - 1]);
-            s_vq[1][lane] = make_double2(vyd[0], vyd[NP - 1]);
-            s_vq[2][lane] = make_double2(vzd[0], vzd[NP - 1]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if constexpr (M64) s_wp[j][lane] = make_double2(wperm[0][j], wperm[NP - 1][j]);
-                else s_wp[j][lane] = make_float2((float)wperm[0][j], (float)wperm[NP - 1][j]);
-            }
-        }
-    }
-    __syncthreads();  // the per-velocity constants in shared memory are complete
-    // uniform coefficients: hoisted (kernel parameters in the single-instance
-    // kernel; FP32 values in registers), except for the FP64 batched kernel,
-    // which re-reads them from shared memory at each use
-    constexpr bool RR = SA && sizeof(T) == 8;
-    const T kz = RR ? T(0) : T(a.c.kz), kx = RR ? T(0) : T(a.c.kx), mu = RR ? T(0) : T(a.c.mu);
-    const T kc = T((R == 3 ? -20.0 : 6.0) * (a.c.kz + a.c.kx));  // centre weight of both axes
-    const T cA0 = RR ? T(0) : T(a.cA), cY0 = RR ? T(0) : T(a.cY);
-    auto K = [&](const double &x, T hoisted) -> T {
-        if constexpr (RR) return T(rd<true>(x));
-        else return hoisted;
-    };
-    const T p2s = T(2 * a.c.pmo * a.c.st), p2c = T(2 * a.c.pmo * a.c.ct), ps = T(a.c.pmo * a.c.st);
-    const bool vac = VAC && a.c.pmo != 0.0;  // batched launches: instances without a vacuum term skip it
-
-    // prime the register queue with planes xs-R .. xs+R-1 (periodic, or from
-    // a slab's halo buffer outside [0, nx))
-    T q[4][W][NP];
-    const T *halo = rd<SA>(a.halo);
-#pragma unroll
-    for (int k = 0; k < 2 * R; ++k) {
-        const int pl = xs - R + k;
-        const bool hal = halo != nullptr && (pl < 0 || pl >= g.nx);
-        const long long o = (long long)wrap_index(pl, g.nx) * P + own;
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            T t[NP];
-            const T *src = hal ? halo + halo_offset(4 * half + f, pl, g.nx, R, P) + own : in + f * fs + o;
-            if (vact) ldv<T, NP>(src, t);
-#pragma unroll
-            for (int p = 0; p < NP; ++p) q[f][k][p] = vact ? t[p] : T(0);
-        }
-    }
-    bool ok = true;
-    if (tid == 0) {  // boxes j < R are only centres: skip those past a short segment's end
-        for (int j = 0; j < R + D && j < nboxes; ++j)
-            if (j >= R || j < nplanes) ok = ok && issue(j);
-        for (int j = 1; j < CF::PFD; ++j) l2pref(j);
-    }
-
-    for (int i = 0; i < nplanes; ++i) {
-        if (tid == 0) {
-            if (ok && i + R + D < nboxes) ok = issue(i + R + D);
-            if (!ok) s_abort = 1;
-            l2pref(i + CF::PFD);
-        }
-        const int x = xs + i;
-        const unsigned ox = (unsigned)x * P32 + own32;  // element offset of (x, zr, v) within a field
-        T uin[4][NP], ain[4][NP];  // U, B
-        {
-            // pointwise epilogue inputs first (they are not in the ring; L2 hits
-            // after the tensor prefetch PFD planes earlier)
-            constexpr bool LU = CF::PU, LA = CF::PA;
-            const T *up = LU ? rd<SA>(a.u) + hoff + ox : nullptr;
-            const T *ap = LA ? rd<SA>(a.acc_src) + hoff + ox : nullptr;
-#pragma unroll
-            for (int f = 0; f < 4; ++f) {
-#pragma unroll
-                for (int p = 0; p < NP; ++p) uin[f][p] = ain[f][p] = T(0);
-                if (vact) {
-                    if (LU) ldv<T, NP>(up + f * fs32, uin[f]);
-                    if (LA) ldv<T, NP>(ap + f * fs32, ain[f]);
-                }
-            }
-        }
-        // the front box (plane i + R) has to be waited for; the centre box was
-        // this warp's front box R planes ago (its slot is not refilled before
-        // its centre use), except for the first R centres, which are never fronts
-        const int jf = i + R, sf = jf % NS, sc = i % NS;
-        if (!mbar_wait(smem_u32(&bars[sf]), (unsigned)((jf / NS) & 1)) ||
-            (i < R && !mbar_wait(smem_u32(&bars[sc]), (unsigned)((i / NS) & 1))) ||
-            ((i & 3) == 0 && *(volatile int *)&s_abort)) {  // another warp's abort, looked at every 4th plane
-            s_abort = 1;
-            break;
-        }
-        const T *fbox = (const T *)(smem + sf * S::bytes + S::box);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) ldv<T, NP>(&fbox[((R + r) * 4 + f) * VB + NP * lane], q[f][2 * R]);
-        if (jf >= nplanes) {  // this box is never a centre: its front use was the last
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bars[NS + sf]));
-        }
-        const unsigned char *sp = smem + sc * S::bytes;
-        const T *zb = (const T *)(sp + S::box);
-        const double *mb = (const double *)(sp + S::mb);
-
-        T sten[4][NP];
-        const T kzp = K(a.c.kz, kz), kxp = K(a.c.kx, kx);
-        T swz[4][NP], swx[4][NP];  // this lane's stencil weights (shared memory, re-read per plane)
-        ldw<T, NP>(&sh.sw[0][lane][0], swz[0], swz[1]);
-        ldw<T, NP>(&sh.sw[1][lane][0], swz[2], swz[3]);
-        ldw<T, NP>(&sh.sw[2][lane][0], swx[0], swx[1]);
-        ldw<T, NP>(&sh.sw[3][lane][0], swx[2], swx[3]);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            T zs[W][NP];
-#pragma unroll
-            for (int k = 0; k < W; ++k)  // the centre row is the x-queue's centre: not re-read
-                if (k != R) ldv<T, NP>(&zb[((r + k) * 4 + f) * VB + NP * lane], zs[k]);
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                T zsp[W], xsp[W], wzp[4], wxp[4];
-#pragma unroll
-                for (int k = 0; k < W; ++k) {
-                    zsp[k] = k == R ? q[f][R][p] : zs[k][p];
-                    xsp[k] = q[f][k][p];
-                }
+            for (int o = 0; o < 2; ++o) {
+                const int vi = (o ? vp : v) + p;
+                const bool in_row = vi < g.nvs;
+                const int vj = in_row ? vi : 0;
+                const double wd = in_row ? a.q.vw[vj] : 0.0;
+                const double v4w[4] = {wd, a.q.vx[vj] * wd, a.q.vy[vj] * wd, a.q.vz[vj] * wd};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    wzp[j] = swz[j][p];
-                    wxp[j] = swx[j][p];
+                    const int k = j ^ wq;
+                    const M w = M(k == 0 ? v4w[0] : k == 1 ? v4w[1] : k == 2 ? v4w[2] : v4w[3]);
+                    if (o) wp[p][j] = w;
+                    else wo[p][j] = w;
                 }
-                const T sz = axis_sum<T, R>(zsp, wzp, kzp), sx = axis_sum<T, R>(xsp, wxp, kxp);
-                sten[f][p] = fma(kc, q[f][R][p], sz + sx);
             }
         }
-        double m[NMOM];
-        {
-            const double2 *m2 = (const double2 *)(mb + r * NMOM);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wz[j] = O::make(tz[j]), wx[j] = O::make(tx[j]);
+    }
+    const V kz = O::splat(a.c.kz), kx = O::splat(a.c.kx), mu = O::splat(a.c.mu);
+    const V kc = O::splat((R == 3 ? -20.0 : 6.0) * (a.c.kz + a.c.kx));  // centre weight of both axes
+    const V cA = O::splat(a.cA), cY = O::splat(a.cY);
+    const V p2s = O::splat(2 * a.c.pmo * a.c.st), p2c = O::splat(2 * a.c.pmo * a.c.ct), ps = O::splat(a.c.pmo * a.c.st);
+    const bool vac = VAC && a.c.pmo != 0.0;  // batched launches: instances without a vacuum term skip it
+
+    // x stencil in transposed form: xs[f][row][k] is the partial sum of the
+    // centre plane (front - R + k) over the planes before the front.  A front
+    // value F completes centre front - R and is added, with its tap's weight,
+    // to the R..2R-1 others; the move to the next slot is the fma's own
+    // destination, so nothing is shifted, and the 2R+1 products of a value are
+    // independent of each other.
+    V sx[4][RW][2 * R];
+    auto tap = [&](int k) -> V {  // weight of a front value in centre (front - R + k)
+        return R == 3 ? (k == 0 || k == 6 ? kx : k == 1 ? wx[3] : k == 2 ? wx[2] : k == 3 ? kc : k == 4 ? wx[1] : wx[0])
+                      : (k == 0 ? wx[3] : k == 1 ? wx[2] : k == 2 ? kc : k == 3 ? wx[1] : wx[0]);
+    };
+    // the planes left of the segment (periodic, or from a slab's halo buffer)
+    {
+        const T *halo = rd<SA>(a.halo);
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+#pragma unroll
+            for (int w = 0; w < RW; ++w)
+#pragma unroll
+                for (int k = 0; k < 2 * R; ++k) sx[f][w][k] = O::zero();
+#pragma unroll
+        for (int b = 0; b < R; ++b) {
+            const int pl = xs - R + b;
+            const bool hal = halo != nullptr && pl < 0;
+            const long long o = (long long)wrap_index(pl, g.nx) * P + own;
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int w = 0; w < RW; ++w) {
+                    const T *src = (hal ? halo + halo_offset(4 * half + f, pl, g.nx, R, P) + own : in + f * fs + o) +
+                                   w * g.nvs;
+                    const V F = vact ? O::ld(src) : O::zero();
+                    auto &q = sx[f][w];
+#pragma unroll
+                    for (int k = 0; k + 1 < 2 * R; ++k) q[k] = vfma(tap(k + 1), F, q[k + 1]);
+                    q[2 * R - 1] = vmul(tap(2 * R), F);
+                }
+        }
+    }
+    // front j of the march: box j's values enter the x sums and, with their z
+    // sums, the centre sum of their own plane; y = the completed stencil sums
+    // of centre j - R
+    auto front = [&](const T *box, V (&y)[4][RW]) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            V zs[2 * R + RW];
+#pragma unroll
+            for (int k = 0; k < 2 * R + RW; ++k) zs[k] = O::ld(&box[((r + k) * 4 + f) * VB + NP * lane]);
+#pragma unroll
+            for (int w = 0; w < RW; ++w) {
+                const V F = zs[R + w];
+                auto &q = sx[f][w];
+                y[f][w] = vfma(tap(0), F, q[0]);
+#pragma unroll
+                for (int k = 0; k + 1 < 2 * R; ++k) q[k] = vfma(tap(k + 1), F, q[k + 1]);
+                q[2 * R - 1] = vmul(tap(2 * R), F);
+                V z = q[R - 1];
+                z = vfma(wz[0], zs[w + R - 2], z);
+                z = vfma(wz[1], zs[w + R - 1], z);
+                z = vfma(wz[2], zs[w + R + 1], z);
+                z = vfma(wz[3], zs[w + R + 2], z);
+                if (R == 3) z = vfma(kz, vadd(zs[w], zs[w + 2 * R]), z);
+                q[R - 1] = z;
+            }
+        }
+    };
+
+    for (int j = 0; j < nboxes; ++j) {
+        const int i = j - R, x = xs + i;  // centre plane completed by front j (none while j < R)
+        const unsigned ox = (unsigned)x * P32 + own32;  // element offset of (x, zr, v) within a field
+        const int sf = j % NS, sc = (j + NS - R) % NS;
+        if (!mbar_wait(smem_u32(&bars[sf]), (unsigned)((j / NS) & 1)) ||
+            ((j & 3) == 0 && *(volatile int *)&sh.abort)) {  // another warp's abort, looked at every 4th plane
+            sh.abort = 1;
+            break;
+        }
+        V y[4][RW];
+        front((const T *)(smem + sf * S::bytes + S::box), y);
+        if (j < R) continue;
+
+        const unsigned char *sp = smem + sc * S::bytes;
+        const T *zb = (const T *)(sp + S::box);
+        V cen[4][RW];
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+#pragma unroll
+            for (int w = 0; w < RW; ++w) cen[f][w] = O::ld(&zb[((r + R + w) * 4 + f) * VB + NP * lane]);
+        V pin[4][RW];  // the pointwise input: U (S2, S3) or B (S4)
+        if (CF::PU || CF::PA) {
+            const T *pb = (const T *)(smem + CF::ring + i % CF::PSM * CF::pbytes);
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int w = 0; w < RW; ++w) pin[f][w] = O::ld(&pb[((r + w) * 4 + f) * VB + NP * lane]);
+        }
+        V outm[4][RW], outb[4][RW];
+#pragma unroll
+        for (int w = 0; w < RW; ++w) {
+            double m[NMOM];
+            const double2 *m2 = (const double2 *)((const double *)(sp + S::mb) + (r + w) * NMOM);
 #pragma unroll
             for (int k = 0; k < NMOM / 2; ++k) {
                 const double2 t = m2[k];
                 m[2 * k] = t.x;
                 m[2 * k + 1] = t.y;
             }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bars[NS + sc]));  // centre use is the box's last use
-
-        T outm[4][NP];
-        double2 vq2[3];
-        if constexpr (kShared) {
+            double ia[NP], ib[NP], ie[NP];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) vq2[c] = s_vq[c][lane];
-        }
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            const double ux = kShared ? (p ? vq2[0].y : vq2[0].x) : vxd[p];
-            const double uy = kShared ? (p ? vq2[1].y : vq2[1].x) : vyd[p];
-            const double uz = kShared ? (p ? vq2[2].y : vq2[2].x) : vzd[p];
-            const T ia = T(inp(m, ux, uy, uz)), ib = T(inp(m + 4, ux, uy, uz)), ie = T(inp(m + 8, ux, uy, uz));
-            const T cen[4] = {q[0][R][p], q[1][R][p], q[2][R][p], q[3][R][p]};
-            const T st4[4] = {sten[0][p], sten[1][p], sten[2][p], sten[3][p]};
-            T kk[4];
-            rhs_half<T, VAC>(cen, ia, ib, ie, K(a.c.mu, mu), p2s, p2c, ps, st4, kk, vac);
-            const T cA = K(a.cA, cA0), cY = K(a.cY, cY0);
+            for (int p = 0; p < NP; ++p) {
+                ia[p] = contract4(m, vx[p], vy[p], vz[p]);
+                ib[p] = contract4(m + 4, vx[p], vy[p], vz[p]);
+                ie[p] = contract4(m + 8, vx[p], vy[p], vz[p]);
+            }
+            // commutator and vacuum terms (nuosc_class.cpp:187-200, 280-287)
+            const V am = vmul(mu, O::make(ia)), bm = vmul(mu, O::make(ib)), em = vmul(mu, O::make(ie));
+            const V ee = cen[0][w], mm = cen[1][w], emr = cen[2][w], emi = cen[3][w];
+            const V nd = vsub(mm, ee);
+            const V h = vfma(emi, am, vmul(emr, bm));
+            V kk[4];
+            kk[0] = vfma(O::splat(2.0), h, y[0][w]);
+            kk[1] = vfma(O::splat(-2.0), h, y[1][w]);
+            kk[2] = vfma(nd, bm, vfma(vneg(em), emi, y[2][w]));
+            kk[3] = vfma(nd, am, vfma(em, emr, y[3][w]));
+            if (VAC && vac) {
+                kk[0] = vfma(vneg(p2s), emi, kk[0]);
+                kk[1] = vfma(p2s, emi, kk[1]);
+                kk[2] = vfma(vneg(p2c), emi, kk[2]);
+                kk[3] = vfma(p2c, emr, vfma(vneg(ps), nd, kk[3]));
+            }
 #pragma unroll
             for (int f = 0; f < 4; ++f) {
+                const V c = cen[f][w];
                 if (MODE == MODE_S1Y) {
-                    outm[f][p] = cen[f] + cY * kk[f];  // Y2
+                    outm[f][w] = vfma(cY, kk[f], c);  // Y2
                 } else if (MODE == MODE_SY) {
-                    outm[f][p] = uin[f][p] + cY * kk[f];  // Y4
+                    outm[f][w] = vfma(cY, kk[f], pin[f][w]);  // Y4
                 } else if (MODE == MODE_S2B) {
-                    const T u = uin[f][p];
-                    ain[f][p] = (u + cen[f]) + cA * kk[f];  // B = U + Y2 + dt k2
-                    outm[f][p] = u + cY * kk[f];            // Y3
+                    const V u = pin[f][w];
+                    outb[f][w] = vfma(cA, kk[f], vadd(u, c));  // B = U + Y2 + dt k2
+                    outm[f][w] = vfma(cY, kk[f], u);          // Y3
                 } else {
-                    outm[f][p] = third_plus(ain[f][p] + cen[f], cA * kk[f]);  // (B + Y4)/3 + dt/6 k4
+                    outm[f][w] = vthird_plus<T>(vadd(pin[f][w], c), vmul(cA, kk[f]));  // (B + Y4)/3 + dt/6 k4
                 }
             }
         }
         if (vact) {
             T *dp = (MODE == MODE_S4B ? rd<SA>(a.acc_dst) : rd<SA>(a.y_dst)) + hoff + ox;
 #pragma unroll
-            for (int f = 0; f < 4; ++f) stv<T, NP>(dp + f * fs32, outm[f]);
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int w = 0; w < RW; ++w) O::st(dp + f * fs32 + w * g.nvs, outm[f][w]);
             if (MODE == MODE_S2B) {
                 T *bp = rd<SA>(a.acc_dst) + hoff + ox;
 #pragma unroll
-                for (int f = 0; f < 4; ++f) stv<T, NP>(bp + f * fs32, ain[f]);
+                for (int f = 0; f < 4; ++f)
+#pragma unroll
+                    for (int w = 0; w < RW; ++w) O::st(bp + f * fs32 + w * g.nvs, outb[f][w]);
             }
         }
-        // velocity-moment partials of the written state (nuosc_class.cpp:69-71):
-        // moment 4c + j = sum over the block's velocities of weight j (w, w vx,
-        // w vy, w vz) times combination c (emr, emi, ee - mm; the neutrino half
-        // enters with sign -1 in combinations 0 and 2, applied to the final
-        // sum, which is exact).
-        // M64 (every FP64 march; the FP32 march when the tile table says so):
-        // products and the warp's reduce-scatter in double -- the float state
-        // converts exactly and each product with a double weight is a double
-        // product, so the sums carry no error beyond the state's own rounding.
-        // FP32 march without M64: in float -- the float state's products with
-        // float-rounded weights, summed over the block's 64 velocities --, the
-        // block's partial stored as double; the blocks and both halves are
-        // summed in FP64 by the finalize either way.
-        // Each lane forms its 12 products (weight slots in its order s ^ wq) and
-        // the warp reduce-scatters them, pairing lanes over bits 4, 3, 2, 1, 0:
-        // over bit 4 weight slots 2 and 3 go to the partner, over bit 3 slot 1,
-        // which leaves every lane the three combinations of weight wq; over bit
-        // 2 the lanes with the bit clear keep combinations 0 and 1, the others
-        // combination 2; over bit 1 the former split 0 and 1 while the latter
-        // sum 2; over bit 0 both sum.  13 shuffle-adds for the 12 sums.
+        // The centre use is the box's last (a right-halo box has none: its slot is
+        // not filled again).  The arrive comes after the stores: they need every
+        // value this plane read from shared memory, so no such read can still be
+        // under way when the producer refills the slots (an arrive that only
+        // follows the loads in program order may overtake them in the pipeline).
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bars[NS + sc]));
         {
-            using M = std::conditional_t<M64, double, float>;
-            M acc[3][4];
-            [[maybe_unused]] std::conditional_t<M64, double2, float2> wp2[kShared ? 4 : 1];
-            if constexpr (kShared) {
+            const bool b4 = lane & 16;
+            T ko[4][NP], kp[4][NP];  // the kept row's values: this lane's velocities, the partner's
 #pragma unroll
-                for (int j = 0; j < 4; ++j) wp2[j] = s_wp[j][lane];
-            }
+            for (int f = 0; f < 4; ++f) {
+                T t0[NP], t1[NP];
+                O::get(outm[f][0], t0);
+                O::get(outm[f][1], t1);
 #pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                const M ee = M(outm[0][p]), mm = M(outm[1][p]), emr = M(outm[2][p]), emi = M(outm[3][p]);
-                const M d[3] = {emr, emi, ee - mm};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    M wj;
-                    if constexpr (kShared) wj = p ? wp2[j].y : wp2[j].x;
-                    else wj = wperm[p][j];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) acc[c][j] = p == 0 ? wj * d[c] : fma(wj, d[c], acc[c][j]);
+                for (int p = 0; p < NP; ++p) {
+                    ko[f][p] = b4 ? t1[p] : t0[p];
+                    if (!M64 || sizeof(T) == 4 || f >= 2) kp[f][p] = __shfl_xor_sync(0xffffffffu, b4 ? t0[p] : t1[p], 16);
+                    else kp[f][p] = b4 ? t0[p] : t1[p];
                 }
             }
+            M acc[3][4];
+#pragma unroll
+            for (int o = 0; o < 2; ++o)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const T *q4[4] = {o ? &kp[0][p] : &ko[0][p], o ? &kp[1][p] : &ko[1][p], o ? &kp[2][p] : &ko[2][p],
+                                      o ? &kp[3][p] : &ko[3][p]};
+                    M dd = M(*q4[0]) - M(*q4[1]);
+                    if (M64 && sizeof(T) == 8 && o) dd = __shfl_xor_sync(0xffffffffu, dd, 16);
+                    const M d[3] = {M(*q4[2]), M(*q4[3]), dd};
+#pragma unroll
+                    for (int jw = 0; jw < 4; ++jw) {
+                        const M w = o ? wp[p][jw] : wo[p][jw];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) acc[c][jw] = o == 0 && p == 0 ? w * d[c] : fma(w, d[c], acc[c][jw]);
+                    }
+                }
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                acc[c][0] += __shfl_xor_sync(0xffffffffu, acc[c][2], 16);
-                acc[c][1] += __shfl_xor_sync(0xffffffffu, acc[c][3], 16);
+                acc[c][0] += __shfl_xor_sync(0xffffffffu, acc[c][2], 8);
+                acc[c][1] += __shfl_xor_sync(0xffffffffu, acc[c][3], 8);
             }
 #pragma unroll
-            for (int c = 0; c < 3; ++c) acc[c][0] += __shfl_xor_sync(0xffffffffu, acc[c][1], 8);
-            const bool b2 = (lane >> 2) & 1, b1 = (lane >> 1) & 1;
-            M k0 = b2 ? acc[2][0] : acc[0][0];
-            k0 += __shfl_xor_sync(0xffffffffu, b2 ? acc[0][0] : acc[2][0], 4);
-            const M k1 = acc[1][0] + __shfl_xor_sync(0xffffffffu, acc[1][0], 4);
-            M kk = (!b2 && b1) ? k1 : k0;
-            kk += __shfl_xor_sync(0xffffffffu, (b2 || b1) ? k0 : k1, 2);
-            kk += __shfl_xor_sync(0xffffffffu, kk, 1);
-            if ((lane & 1) == 0 && !(b2 && b1)) {  // lanes 0 mod 2 hold moment 4c + wq
-                const int c = b2 ? 2 : (int)b1;
+            for (int c = 0; c < 3; ++c) acc[c][0] += __shfl_xor_sync(0xffffffffu, acc[c][1], 4);
+            const bool b1 = (lane >> 1) & 1, b0 = lane & 1;
+            M k0 = b1 ? acc[2][0] : acc[0][0];
+            k0 += __shfl_xor_sync(0xffffffffu, b1 ? acc[0][0] : acc[2][0], 2);
+            const M k1 = acc[1][0] + __shfl_xor_sync(0xffffffffu, acc[1][0], 2);
+            M kk = (!b1 && b0) ? k1 : k0;
+            kk += __shfl_xor_sync(0xffffffffu, (b1 || b0) ? k0 : k1, 1);
+            if (!(b1 && b0)) {  // lane holds moment 4c + wq of its kept row
+                const int c = b1 ? 2 : (int)b0;
                 const double v = (double)kk;
-                const unsigned cell = (unsigned)x * (unsigned)rd<SA>(a.g.nz) + (unsigned)zr;
+                const unsigned cell = (unsigned)x * (unsigned)rd<SA>(a.g.nz) + (unsigned)(zr + (b4 ? 1 : 0));
                 rd<SA>(a.mom_part)[((cell * (unsigned)nvb + (unsigned)vb) * 2u + (unsigned)half) * NMOM + 4 * c + wq] =
                     (half || c == 1) ? v : -v;
             }
         }
-#pragma unroll
-        for (int f = 0; f < 4; ++f)
-#pragma unroll
-            for (int k = 0; k < 2 * R; ++k)
-#pragma unroll
-                for (int p = 0; p < NP; ++p) q[f][k][p] = q[f][k + 1][p];
     }
     __syncthreads();
-    const bool aborted = s_abort != 0;
-    if (tid == 0) {
-        if (aborted) {
-            // a wait expired: report it, then wait (bounded) for the copies of
-            // the last NS boxes issued -- the only ones that may still be in
-            // flight: box j - NS of a slot was consumed (so had landed) before
-            // box j was issued into it -- before the CTA's shared memory is
-            // reused or released
-            atomicExch(a.status, NUOSC_TIMEOUT_CODE);
-            for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
-                if (j >= R || j < nplanes) mbar_wait(smem_u32(&bars[j % NS]), (unsigned)((j / NS) & 1));
-        }
-        for (int s = 0; s < 2 * NS; ++s) mbar_inval(smem_u32(&bars[s]));
-    }
-    return aborted;
+    return sh.abort != 0;
 }
 
 // grid (velocity blocks run by this kernel, z tiles, 2 x x-segments); nvb:
 // velocity blocks of the moment partials (one more when a tail kernel runs
 // the last block)
 template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
-__global__ void __launch_bounds__(32 * TZ, tma_ctas_per_sm<T, TZ>())
+__global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
     k_xtma(const __grid_constant__ TmaMaps maps, const StageArgs<T> a, int LX, int nvb) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ MarchShared<T, M64> sh;
+    __shared__ MarchShared sh;
     const int xs = (blockIdx.z >> 1) * LX;
     if (xs >= a.g.nx) return;
-    const TmaMaps *mp = &maps;
-    xtma_march<T, R, MODE, TZ, VAC, false, M64>(mp, a, blockIdx.y * TZ, blockIdx.x, nvb, xs, min(xs + LX, a.g.nx),
-                                           blockIdx.z & 1, smem, sh);
+    const Tile t{(int)blockIdx.y * TZ, (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx), (int)blockIdx.z & 1};
+    if (threadIdx.x >= 32 * (TZ / RW)) {
+        setmaxnreg_dec<RegSplit<TZ>::producer>();
+        xtma_produce<T, R, MODE, TZ, M64>(maps, a, t, smem, sh);
+    } else {
+        setmaxnreg_inc<RegSplit<TZ>::consumer>();
+        xtma_consume<T, R, MODE, TZ, VAC, false, M64>(a, t, smem, sh);
+    }
 }
 
 // One instance's stage in a batched launch: its tensor maps (over the stage's
@@ -733,63 +761,74 @@ struct __align__(64) BatchItem {
 // the vacuum term in (for batches with any pmo != 0); it is then switched per
 // instance at run time.
 template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
-__global__ void __launch_bounds__(32 * TZ, tma_ctas_per_sm<T, TZ>())
+__global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
     k_xtma_batch(const BatchItem<T> *items, const long long *__restrict__ starts, int ninst, long long nitems,
                  unsigned long long *counter, const int *__restrict__ halt) {
     constexpr int NW = (int)(sizeof(StageArgs<T>) / 8);
-    static_assert(sizeof(StageArgs<T>) % 8 == 0 && NW <= 32 * TZ, "StageArgs copy: one 8-byte word per thread");
+    constexpr int NC = 32 * (TZ / RW);  // consumer threads
+    static_assert(sizeof(StageArgs<T>) % 8 == 0 && NW <= 128, "StageArgs copy: one 8-byte word per producer thread");
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ MarchShared<T, M64> sh;
+    __shared__ MarchShared sh;
     __shared__ __align__(16) StageArgs<T> s_a;
     __shared__ const TmaMaps *s_mp;
-    __shared__ int s_t[6];  // instance (-1: no tiles left, -2: a stopped instance's tile), z0, vb, xs, xe, half
-    for (;;) {
-        __syncthreads();  // every thread is done with the previous tile's arguments
-        if (threadIdx.x == 0) {
-            const long long it = (long long)atomicAdd(counter, 1ull);
-            s_t[0] = -1;
-            if (it < nitems) {
-                int lo = 0, hi = ninst - 1;  // last instance whose first tile is <= it
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (starts[mid] <= it) lo = mid;
-                    else hi = mid - 1;
+    __shared__ Tile s_t;
+    __shared__ int s_inst;  // instance (-1: no tiles left, -2: a stopped instance's tile)
+    if (threadIdx.x >= NC) {
+        setmaxnreg_dec<RegSplit<TZ>::producer>();
+        for (;;) {
+            __syncthreads();  // every thread is done with the previous tile's arguments
+            if (threadIdx.x == NC) {
+                const long long it = (long long)atomicAdd(counter, 1ull);
+                s_inst = -1;
+                if (it < nitems) {
+                    int lo = 0, hi = ninst - 1;  // last instance whose first tile is <= it
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (starts[mid] <= it) lo = mid;
+                        else hi = mid - 1;
+                    }
+                    const BatchItem<T> &e = items[lo];
+                    int loc = (int)(it - starts[lo]);  // ((seg * 2 + half) * ntz + zt) * nvbm + vb
+                    s_inst = (halt && halt[lo]) ? -2 : lo;
+                    s_t.vb = loc % e.nvbm;
+                    loc /= e.nvbm;
+                    s_t.z0 = loc % e.ntz * TZ;
+                    loc /= e.ntz;
+                    s_t.half = loc & 1;
+                    s_t.xs = (loc >> 1) * e.lx;
+                    s_t.xe = min(s_t.xs + e.lx, e.a.g.nx);
+                    s_t.nvb = e.nvb;
+                    s_mp = &e.maps;
+                    // this thread issues every TMA load of the tile; the maps were written
+                    // through the generic proxy (a host copy when the work-list was built)
+                    tensormap_acquire(&e.maps.zr);
+                    tensormap_acquire(&e.maps.tzr);
+                    tensormap_acquire(&e.maps.tz);
+                    tensormap_acquire(&e.maps.r);
+                    if (MarchCfg<T, R, MODE, TZ>::PU) tensormap_acquire(&e.maps.pu);
+                    if (MarchCfg<T, R, MODE, TZ>::PA) tensormap_acquire(&e.maps.pa);
                 }
-                const BatchItem<T> &e = items[lo];
-                long long loc = it - starts[lo];  // ((seg * 2 + half) * ntz + zt) * nvbm + vb
-                s_t[0] = (halt && halt[lo]) ? -2 : lo;
-                const int vb = (int)(loc % e.nvbm);
-                loc /= e.nvbm;
-                const int zt = (int)(loc % e.ntz);
-                loc /= e.ntz;
-                const int xs = (int)(loc >> 1) * e.lx;
-                s_t[1] = zt * TZ;
-                s_t[2] = vb;
-                s_t[3] = xs;
-                s_t[4] = min(xs + e.lx, e.a.g.nx);
-                s_t[5] = (int)(loc & 1);
-                s_mp = &e.maps;
-                // thread 0 issues every TMA load of the tile; the maps were written
-                // through the generic proxy (a host copy when the work-list was built)
-                tensormap_acquire(&e.maps.zr);
-                tensormap_acquire(&e.maps.tzr);
-                tensormap_acquire(&e.maps.tz);
-                tensormap_acquire(&e.maps.r);
-                if (MarchCfg<T, R, MODE, TZ>::PU) tensormap_acquire(&e.maps.pu);
-                if (MarchCfg<T, R, MODE, TZ>::PA) tensormap_acquire(&e.maps.pa);
             }
+            __syncthreads();
+            const int lo = s_inst;
+            if (lo == -1) break;
+            if (lo == -2) continue;  // every thread: the loop's first barrier comes next
+            const int w = threadIdx.x - NC;
+            if (w < NW) reinterpret_cast<long long *>(&s_a)[w] = reinterpret_cast<const long long *>(&items[lo].a)[w];
+            __syncthreads();  // s_a is complete
+            if (xtma_produce<T, R, MODE, TZ, M64>(*s_mp, s_a, s_t, smem, sh)) break;
         }
-        __syncthreads();
-        const int lo = s_t[0];
-        if (lo == -1) break;
-        if (lo == -2) continue;  // every thread: the loop's first barrier comes next
-        if (threadIdx.x < NW)
-            reinterpret_cast<long long *>(&s_a)[threadIdx.x] =
-                reinterpret_cast<const long long *>(&items[lo].a)[threadIdx.x];
-        const int nvb = items[lo].nvb;
-        const int z0 = s_t[1], vb = s_t[2], xs = s_t[3], xe = s_t[4], half = s_t[5];
-        __syncthreads();  // s_a is complete
-        if (xtma_march<T, R, MODE, TZ, VAC, true, M64>(s_mp, s_a, z0, vb, nvb, xs, xe, half, smem, sh)) break;
+    } else {
+        setmaxnreg_inc<RegSplit<TZ>::consumer>();
+        for (;;) {
+            __syncthreads();
+            __syncthreads();
+            const int lo = s_inst;
+            if (lo == -1) break;
+            if (lo == -2) continue;
+            __syncthreads();
+            if (xtma_consume<T, R, MODE, TZ, VAC, true, M64>(s_a, s_t, smem, sh)) break;
+        }
     }
 }
 
@@ -881,7 +920,7 @@ bool make_maps(TmaMaps *m, const StageArgs<T> &a, int tz, int r) {
 template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
 cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     using CF = MarchCfg<T, R, MODE, TZ>;
-    static_assert(tma_ctas_per_sm<T, TZ>() * (CF::smem + sizeof(MarchShared<T, M64>) + 64 + 1024) <= 228 * 1024,
+    static_assert(tma_ctas_per_sm<T, TZ>() * (CF::smem + sizeof(MarchShared) + sizeof(StageArgs<T>) + 64 + 1024) <= 228 * 1024,
                   "ring exceeds shared memory");
     TmaMaps maps;
     if (!make_maps<T>(&maps, a, TZ, R)) return cudaErrorInvalidValue;
@@ -895,7 +934,7 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     // velocity blocks fastest: the CTAs resident at once read whole velocity
     // rows of a few z rows (DRAM page locality) rather than one block of many rows
     dim3 grid(nvbm, a.g.nz / TZ, nseg * 2);
-    k_xtma<T, R, MODE, TZ, VAC, M64><<<grid, 32 * TZ, smem, s>>>(maps, a, t.lx, nvb);
+    k_xtma<T, R, MODE, TZ, VAC, M64><<<grid, threads_of(TZ), smem, s>>>(maps, a, t.lx, nvb);
     return cudaGetLastError();
 }
 
@@ -936,7 +975,7 @@ int batch_grid_t(int device) {
     auto kern = k_xtma_batch<T, R, MODE, TZ, VAC, M64>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
     int per_sm = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * TZ, smem) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads_of(TZ), smem) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || per_sm < 1)
         return -1;
     return per_sm * sms;
@@ -945,7 +984,7 @@ int batch_grid_t(int device) {
 template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
 cudaError_t batch_launch_t(const void *items, const long long *starts, int n, long long ntiles,
                            unsigned long long *counter, const int *halt, int grid, cudaStream_t s) {
-    k_xtma_batch<T, R, MODE, TZ, VAC, M64><<<grid, 32 * TZ, batch_smem<T, R, MODE, TZ>(), s>>>(
+    k_xtma_batch<T, R, MODE, TZ, VAC, M64><<<grid, threads_of(TZ), batch_smem<T, R, MODE, TZ>(), s>>>(
         (const BatchItem<T> *)items, starts, n, ntiles, counter, halt);
     return cudaGetLastError();
 }
