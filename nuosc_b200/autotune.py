@@ -4,7 +4,7 @@ velocity-moment summation.
     python -m nuosc_b200.autotune --nn 8 --precision 0 --size 1024 [--write]
 
 For one (velocity count, precision) it times full RK4 steps for every
-candidate tile (tz z-rows per CTA in {4, 8, 16} -- 32 tz threads per CTA --,
+candidate tile (tz z-rows per CTA in {4, 8, 16},
 lx x-planes per CTA) with CUDA events on the solver's stream.  In FP32 it then
 times the best tile with each way of summing the moment partials of a
 velocity block (msum 1: FP64 products and sums; 0: float) and measures each
@@ -12,7 +12,9 @@ one's summation error (NuOsc.moment_error: the fused cell moments against an
 FP64 recomputation from the same stored state); it keeps the fastest whose
 error is within MSUM_TOL.  With --write the choice goes to
 nuosc_b200/tiles.txt ("nv precision tz lx kernel msum" per line), which the
-library reads when a handle is created.  The direct kernel is timed too, for
+library reads when a handle is created (lx 0 there, as in the table that comes
+with the library, leaves the segment length to a rule on the grid).  The direct
+kernel is timed too, for
 reference.  Results are printed as one JSON line.
 
 The velocity block of the TMA kernel is not a tuning dimension: it is one

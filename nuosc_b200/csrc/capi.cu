@@ -96,6 +96,7 @@ struct nuosc_handle {
     double n_nue0[2] = {0, 0};
     int kernel = NUOSC_KERNEL_AUTO;
     XTile tile{16, 64, 32};
+    bool auto_lx = false;    // tile.lx is xtma_lx's choice for this grid alone
     long long launches = 0;
     bool mom_valid = false;  // d_mom holds the moments of v_stat
     unsigned fault_tx = 0;   // self-test of the TMA kernels' bounded waits (nuosc_selftest_overdeclare_tx)
@@ -371,7 +372,20 @@ int stage_path(nuosc_handle *h, XTile &tile) {
     case NUOSC_KERNEL_XTMA: return tma ? 2 : -1;
     default:
         if (h->tile.kind == NUOSC_KERNEL_XMARCH && cpa) return 1;
-        return tma ? 2 : cpa ? 1 : 0;
+        if (tma) return 2;
+        // nz is no multiple of 8: the TMA kernel with overlapping z tiles
+        if (!h->halo) {
+            for (int tz : {16, 8}) {
+                XTile t = h->tile;
+                if (t.tz < tz) continue;
+                t.tz = tz;
+                if (xtma_fits<T>(h->g, t)) {
+                    tile = t;
+                    return 2;
+                }
+            }
+        }
+        return cpa ? 1 : 0;
     }
 }
 
@@ -517,7 +531,7 @@ int step_impl(nuosc_handle *h, int nsteps) {
 template <typename T>
 int stage_impl(nuosc_handle *h, int k) {
     XTile tile;
-    if (stage_path<T>(h, tile) != 2)
+    if (stage_path<T>(h, tile) != 2 || h->g.nz % tile.tz)
         return fail(NUOSC_ERR_UNSUPPORTED, "nuosc_stage runs the TMA stage kernel, which does not take this geometry");
     const size_t need = (size_t)h->g.ncell * xmarch_num_vblocks(h->g, h->tile) * 2 * NMOM * sizeof(double);
     if (int rc = ensure((void **)&h->d_part, &h->part_bytes, need, h)) return rc;
@@ -865,6 +879,14 @@ int nuosc_create(const nuosc_params *p, nuosc_handle **out) {
     };
     cudaError_t e = cudaSetDevice(h->device);
     if (e != cudaSuccess) return bail(fail(NUOSC_ERR_CUDA, "cudaSetDevice(%d): %s", h->device, cudaGetErrorString(e)));
+    if (h->tile.lx == 0) {
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+        // the step falls back to 8-row tiles where 16 rows do not fit
+        const int tz = h->tile.tz == 16 && nz < 22 ? 8 : h->tile.tz;
+        h->tile.lx = h->precision == NUOSC_FP64 ? xtma_lx<double>(h->g, tz, sms) : xtma_lx<float>(h->g, tz, sms);
+        h->auto_lx = true;
+    }
     e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(fail(NUOSC_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e)));
     const size_t reg_bytes = (size_t)h->g.fs * NF * h->esize;
@@ -997,6 +1019,7 @@ int nuosc_set_tile(nuosc_handle *h, int tz, int lx) {
     const int nvb_old = xmarch_num_vblocks(h->g, h->tile);
     h->tile.tz = tz;
     h->tile.lx = lx;
+    h->auto_lx = false;
     if (xmarch_num_vblocks(h->g, h->tile) != nvb_old) h->mom_valid = false;
     return NUOSC_OK;
 }
@@ -1610,7 +1633,10 @@ int batch_build(nuosc_batch *b) {
         };
         long long total = 0;
         for (int i = 0; i < n; ++i) {
-            lxs[i] = std::min(b->m[i]->tile.lx, b->m[i]->g.nx);  // (the same single segment)
+            // a lone solve's automatic length splits its grid over the whole
+            // device; a member starts from long segments
+            const int lx = b->m[i]->auto_lx ? 128 : b->m[i]->tile.lx;
+            lxs[i] = std::min(lx, b->m[i]->g.nx);  // (the same single segment)
             total += tiles_of(i, lxs[i]);
         }
         while (total < target) {

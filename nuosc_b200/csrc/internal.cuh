@@ -114,7 +114,7 @@ cudaError_t launch_stage_direct(const StageArgs<T> &a, int mode, bool ko6, cudaS
 // x-march kernel: tile shape chosen by the autotuner (tile.cu)
 struct XTile {
     int tz;        // z rows per CTA
-    int lx;        // x planes marched per CTA
+    int lx;        // x planes marched per CTA (0 in the tile table: xtma_lx picks it for the grid)
     int vb;        // velocities per CTA (32)
     int kind = 0;  // preferred x-march kernel from the tile table: 2 cp.async, 3 TMA, 0 either
     int msum = 1;  // FP32 TMA march: moment partials summed in FP64 (1) or in float within a block (0)
@@ -123,9 +123,16 @@ template <typename T>
 bool xmarch_supported(const Geom &g, bool ko6, XTile t);
 template <typename T>
 cudaError_t launch_stage_xmarch(const StageArgs<T> &a, int mode, bool ko6, XTile t, cudaStream_t s);
-// TMA-fed variant of the x-march kernel (xtma.cu); needs nz % tz == 0
+// TMA-fed variant of the x-march kernel (xtma.cu).  fits: it runs this grid
+// (nz >= tz + 6); supported: and nz % tz == 0, which batches, x-slabs and an
+// explicitly requested TMA kernel need
+template <typename T>
+bool xtma_fits(const Geom &g, XTile t);
 template <typename T>
 bool xtma_supported(const Geom &g, XTile t);
+// x planes per CTA for grid g on a device of `sms` SMs
+template <typename T>
+int xtma_lx(const Geom &g, int tz, int sms);
 template <typename T>
 cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, cudaStream_t s);
 // velocity blocks of the TMA kernel's moment partials (32 velocities per block in FP64, 64 in FP32)

@@ -435,7 +435,8 @@ template cudaError_t launch_stage_xmarch<float>(const StageArgs<float> &, int, b
 // Tile table keyed on (velocity count, precision): lines "nv precision tz lx
 // [kernel]" in tiles.txt beside the library (or the file named by
 // NUOSC_TILES), written by the autotuner nuosc_b200/autotune.py; kernel 2 is
-// the cp.async x-march, 3 the TMA one.  Shapes not listed use 16 x 128.
+// the cp.async x-march, 3 the TMA one; lx 0 leaves the segment length to
+// xtma_lx.  Shapes not listed use 16-row tiles and xtma_lx.
 XTile autotune_lookup(int nv, int precision) {
     static std::vector<std::array<int, 6>> table;
     static std::once_flag once;
@@ -463,9 +464,9 @@ XTile autotune_lookup(int nv, int precision) {
         fclose(f);
     });
     for (const auto &e : table)
-        if (e[0] == nv && e[1] == precision && (e[2] == 4 || e[2] == 8 || e[2] == 16) && e[3] >= 1)
+        if (e[0] == nv && e[1] == precision && (e[2] == 4 || e[2] == 8 || e[2] == 16) && e[3] >= 0)
             return XTile{e[2], e[3], VB, e[4], e[5] != 0};
-    return XTile{16, 128, VB, 0, 1};
+    return XTile{16, 0, VB, 0, 1};
 }
 
 }  // namespace nuosc

@@ -31,7 +31,7 @@
 //     stop test) has its tiles skipped.
 // All mbarrier waits are bounded: on expiry the kernel records the timeout in
 // the status word, stops marching and, before returning, waits (again
-// bounded) for the copies it issued.  Requires nz % TZ == 0.
+// bounded) for the copies it issued.  nz need not be a multiple of TZ (tile_z0).
 //
 // What bounds it, measured on a 512 x 256 x 642 FP64 grid (KO6): S1 2.8 ms (2
 // state passes, 3.9 TB/s) is held by instruction latency at 8 consumer warps
@@ -312,6 +312,14 @@ __device__ __forceinline__ P rd(const P &x) {
     else return x;
 }
 
+// First row of z tile zt of ntz.  Where TZ does not divide nz, the ntz =
+// ceil(nz / TZ) tiles are spread evenly and overlap: rows of two tiles are
+// computed twice, to the same bits (no stage writes what it reads).  With nz >=
+// TZ + 6 neighbouring tiles are at least 3 >= R rows apart, so only the first
+// and the last tile's box crosses the periodic end and the box pieces are those
+// of an exact division.
+__device__ __forceinline__ int tile_z0(int zt, int ntz, int nz, int tz) { return zt * (nz - tz) / (ntz - 1); }
+
 // One tile of work: z rows z0..z0+TZ-1, velocity block vb (of nvb), x planes
 // xs..xe-1, flavour half `half`
 struct Tile {
@@ -431,7 +439,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     const int v = vb * VB + NP * lane;  // first of this thread's NP velocities
     const bool vact = v < g.nvs;        // nvs is a multiple of NP, so all NP are active together
     const int nplanes = t.xe - xs, nboxes = nplanes + R;
-    const int zr = z0 + r;  // < nz since nz % TZ == 0
+    const int zr = z0 + r;  // < nz
     const long long fs = g.fs;
     const long long P = (long long)g.nz * g.nvs;
     const long long hoff = (long long)half * 4 * fs;
@@ -726,7 +734,7 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
     __shared__ MarchShared sh;
     const int xs = (blockIdx.z >> 1) * LX;
     if (xs >= a.g.nx) return;
-    const Tile t{(int)blockIdx.y * TZ, (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx), (int)blockIdx.z & 1};
+    const Tile t{tile_z0(blockIdx.y, gridDim.y, a.g.nz, TZ), (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx), (int)blockIdx.z & 1};
     if (threadIdx.x >= 32 * (TZ / RW)) {
         setmaxnreg_dec<RegSplit<TZ>::producer>();
         xtma_produce<T, R, MODE, TZ, M64>(maps, a, t, smem, sh);
@@ -933,7 +941,7 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     if (nvbm < 1) return cudaSuccess;  // the tail kernel runs every velocity
     // velocity blocks fastest: the CTAs resident at once read whole velocity
     // rows of a few z rows (DRAM page locality) rather than one block of many rows
-    dim3 grid(nvbm, a.g.nz / TZ, nseg * 2);
+    dim3 grid(nvbm, (a.g.nz + TZ - 1) / TZ, nseg * 2);
     k_xtma<T, R, MODE, TZ, VAC, M64><<<grid, threads_of(TZ), smem, s>>>(maps, a, t.lx, nvb);
     return cudaGetLastError();
 }
@@ -1021,13 +1029,44 @@ struct BatchLaunch {
 }  // namespace
 
 template <typename T>
-bool xtma_supported(const Geom &g, XTile t) {
+bool xtma_fits(const Geom &g, XTile t) {
     // nz >= tz + 6: the widest box (tz + 2R rows, R <= 3) fits in the z extent;
     // 3 fs < 2^32: the march's per-plane offsets within a flavour half are
     // 32-bit (registers of up to 91 GB in FP64, 45 GB in FP32: every state
     // whose four registers fit a B200)
-    return (t.tz == 8 || t.tz == 16) && g.nz % t.tz == 0 && g.nz >= t.tz + 6 && g.nx >= 4 &&
+    return (t.tz == 8 || t.tz == 16) && g.nz >= t.tz + 6 && g.nx >= 4 &&
            g.nvs % vpt<T>() == 0 && 3 * g.fs < (1ll << 32) && encode_fn() != nullptr;
+}
+
+template <typename T>
+bool xtma_supported(const Geom &g, XTile t) {
+    return g.nz % t.tz == 0 && xtma_fits<T>(g, t);
+}
+
+// x planes per CTA.  A segment costs its planes plus about 10 more (the launch of
+// the CTA, the constants, R planes left of it and R right of it), and a launch
+// costs whole waves of CTAs, so the number of segments minimises waves x (lx +
+// 10); among segment counts within 2 % the fewest.  Measured (us per FP64 step,
+// best of a sweep over lx in brackets): 32x32x42 lx 2: 53 [53], 16: 109, 32:
+// 174; 64x64x162 lx 22: 208 [208], 32: 238, 64: 371; 128x128x162 lx 43: 570
+// [566], 32: 636, 64: 749; 128x128x642 lx 64: 1817 [1817], 128: 2015;
+// 100x90x162 lx 50: 344 [344], 34: 426, 100: 525; from 512x256x642 on every lx
+// from 40 to 256 is within 2 %.
+template <typename T>
+int xtma_lx(const Geom &g, int tz, int sms) {
+    const long long slots = (long long)sms * (tz == 16 ? 1 : 2);
+    const long long per = (long long)((g.nz + tz - 1) / tz) * march_vblocks<T>(g) * 2;  // CTAs per segment
+    int best = g.nx;
+    double cost = -1.0;
+    for (int n = 1; n <= g.nx; ++n) {
+        const int lx = (g.nx + n - 1) / n, nseg = (g.nx + lx - 1) / lx;
+        const double c = (double)((per * nseg + slots - 1) / slots) * (lx + 10);
+        if (cost < 0.0 || c < 0.98 * cost) {
+            cost = c;
+            best = lx;
+        }
+    }
+    return best;
 }
 
 template <typename T>
@@ -1089,12 +1128,16 @@ int xtma_tail_v0(const Geom &g) {
 
 template <typename T>
 cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, cudaStream_t s) {
-    if (!a.mom_part || a.g.nz % t.tz) return cudaErrorInvalidValue;
+    if (!a.mom_part || !xtma_fits<T>(a.g, t)) return cudaErrorInvalidValue;
     if (t.tz == 16) return ko6 ? launch_tms<T, 3, 16>(a, mode, t, s) : launch_tms<T, 2, 16>(a, mode, t, s);
     return ko6 ? launch_tms<T, 3, 8>(a, mode, t, s) : launch_tms<T, 2, 8>(a, mode, t, s);
 }
 
 template bool xtma_supported<double>(const Geom &, XTile);
+template bool xtma_fits<double>(const Geom &, XTile);
+template int xtma_lx<double>(const Geom &, int, int);
+template int xtma_lx<float>(const Geom &, int, int);
+template bool xtma_fits<float>(const Geom &, XTile);
 template bool xtma_supported<float>(const Geom &, XTile);
 template int xtma_num_vblocks<double>(const Geom &);
 template int xtma_num_vblocks<float>(const Geom &);
