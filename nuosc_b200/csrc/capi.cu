@@ -301,7 +301,11 @@ int run_stage_direct(nuosc_handle *h, int mode, int in, int u, int acc_src, int 
         h->launches++;
     }
     const int ps = h->prof_begin(prof_kind(mode));
-    CUDA_TRY(launch_stage_direct<T>(a, mode, h->ko6, h->stream));
+    if (mode == MODE_RHS && (h->kernel == NUOSC_KERNEL_AUTO || h->kernel == NUOSC_KERNEL_XTMA) &&
+        rhs_xtma_fits<T>(h->g, a.in, a.acc_dst))
+        CUDA_TRY(launch_rhs_xtma<T>(a, h->ko6, h->stream));  // (and its tail, when there is one)
+    else
+        CUDA_TRY(launch_stage_direct<T>(a, mode, h->ko6, h->stream));
     h->prof_end(ps);
     h->launches++;
     return 0;

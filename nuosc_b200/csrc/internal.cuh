@@ -135,6 +135,12 @@ template <typename T>
 int xtma_lx(const Geom &g, int tz, int sms);
 template <typename T>
 cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, cudaStream_t s);
+// calRHS (MODE_RHS: acc_dst = L(in), mom_in = the moments of in) on the TMA
+// march, for grids and buffers it fits
+template <typename T>
+bool rhs_xtma_fits(const Geom &g, const void *in, const void *out);
+template <typename T>
+cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, cudaStream_t s);
 // velocity blocks of the TMA kernel's moment partials (32 velocities per block in FP64, 64 in FP32)
 template <typename T>
 int xtma_num_vblocks(const Geom &g);

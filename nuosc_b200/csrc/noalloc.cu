@@ -12,8 +12,9 @@
 // of up to NUOSC_NOALLOC_MAX_CELLS cells.  Every GPU that loads the library
 // holds that array (6 MiB) until the process exits.
 //
-// The kernels are the library's own moment pass and direct stage kernel
-// (kernels.cu), unchanged; only the scratch pointer differs.
+// The kernels are the library's own moment pass (kernels.cu) and the TMA march
+// (xtma.cu) -- or the direct stage kernel, for grids with nz < 14 and buffers
+// whose rows are not 16-byte aligned; only the scratch pointer differs.
 #include "../../include/nuosc_b200.h"
 #include "internal.cuh"
 
@@ -141,7 +142,9 @@ extern "C" int nuosc_calrhs_noalloc(const nuosc_rhs_desc *d, const void *in, voi
         a.c = c;
         a.cA = 1.0;
         e = launch_moments<double>(a.in, scratch, q, g, s);
-        if (e == cudaSuccess) e = launch_stage_direct<double>(a, MODE_RHS, ko6, s);
+        if (e == cudaSuccess)
+            e = rhs_xtma_fits<double>(g, in, out) ? launch_rhs_xtma<double>(a, ko6, s)
+                                                  : launch_stage_direct<double>(a, MODE_RHS, ko6, s);
     } else {
         StageArgs<float> a{};
         a.in = (const float *)in;
@@ -152,7 +155,9 @@ extern "C" int nuosc_calrhs_noalloc(const nuosc_rhs_desc *d, const void *in, voi
         a.c = c;
         a.cA = 1.0;
         e = launch_moments<float>(a.in, scratch, q, g, s);
-        if (e == cudaSuccess) e = launch_stage_direct<float>(a, MODE_RHS, ko6, s);
+        if (e == cudaSuccess)
+            e = rhs_xtma_fits<float>(g, in, out) ? launch_rhs_xtma<float>(a, ko6, s)
+                                                 : launch_stage_direct<float>(a, MODE_RHS, ko6, s);
     }
     if (e != cudaSuccess) return fail(NUOSC_ERR_CUDA, cudaGetErrorString(e));
     return NUOSC_OK;

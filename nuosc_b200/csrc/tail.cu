@@ -81,7 +81,9 @@ __device__ __forceinline__ void tail_point(const StageArgs<T> &a, const long lon
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
             const long long idx = o + f * g.fs;
-            if (MODE == MODE_S1Y) {
+            if (MODE == MODE_RHS) {
+                a.acc_dst[idx] = kv[f];
+            } else if (MODE == MODE_S1Y) {
                 outm[f] = c4[f] + cY * kv[f];  // Y2
                 a.y_dst[idx] = outm[f];
             } else if (MODE == MODE_SY) {
@@ -99,23 +101,27 @@ __device__ __forceinline__ void tail_point(const StageArgs<T> &a, const long lon
         }
         // velocity-moment contributions (nuosc_class.cpp:69-71): moment 4c + j
         // = weight j (w, w vx, w vy, w vz) x combination c of the half
-        const double w4[4] = {wd, vxd * wd, vyd * wd, vzd * wd};
-        double d[3];
-        if (half == 0) moment_terms<false>(outm[0], outm[1], outm[2], outm[3], d[0], d[1], d[2]);
-        else moment_terms<true>(outm[0], outm[1], outm[2], outm[3], d[0], d[1], d[2]);
+        if constexpr (MODE != MODE_RHS) {  // (calRHS writes no state)
+            const double w4[4] = {wd, vxd * wd, vyd * wd, vzd * wd};
+            double d[3];
+            if (half == 0) moment_terms<false>(outm[0], outm[1], outm[2], outm[3], d[0], d[1], d[2]);
+            else moment_terms<true>(outm[0], outm[1], outm[2], outm[3], d[0], d[1], d[2]);
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int jw = 0; jw < 4; ++jw) mom[4 * c + jw] = w4[jw] * d[c];
+                for (int jw = 0; jw < 4; ++jw) mom[4 * c + jw] = w4[jw] * d[c];
+        }
     }
-    // sum over the lanes of the (cell, half) (xor offsets below twp stay inside its group)
-    for (int off = twp >> 1; off > 0; off >>= 1)
+    if constexpr (MODE != MODE_RHS) {
+        // sum over the lanes of the (cell, half) (xor offsets below twp stay inside its group)
+        for (int off = twp >> 1; off > 0; off >>= 1)
 #pragma unroll
-        for (int k = 0; k < NMOM; ++k) mom[k] += __shfl_xor_sync(0xffffffffu, mom[k], off);
-    if (lane_in_cell == 0 && cell < g.ncell) {
-        double *p = a.mom_part + ((cell * nvb + (nvb - 1)) * 2 + half) * NMOM;
+            for (int k = 0; k < NMOM; ++k) mom[k] += __shfl_xor_sync(0xffffffffu, mom[k], off);
+        if (lane_in_cell == 0 && cell < g.ncell) {
+            double *p = a.mom_part + ((cell * nvb + (nvb - 1)) * 2 + half) * NMOM;
 #pragma unroll
-        for (int k = 0; k < NMOM; ++k) p[k] = mom[k];
+            for (int k = 0; k < NMOM; ++k) p[k] = mom[k];
+        }
     }
 }
 
@@ -160,6 +166,7 @@ cudaError_t launch_tail_ko(const StageArgs<T> &a, int mode, int v0, int twp, int
     const long long threads = a.g.ncell * 2 * twp;
     const unsigned blocks = (unsigned)((threads + TAIL_BLOCK - 1) / TAIL_BLOCK);
     switch (mode) {
+    case MODE_RHS: k_stage_tail<T, KO6, MODE_RHS><<<blocks, TAIL_BLOCK, 0, s>>>(a, v0, twp, nvb); break;
     case MODE_S1Y: k_stage_tail<T, KO6, MODE_S1Y><<<blocks, TAIL_BLOCK, 0, s>>>(a, v0, twp, nvb); break;
     case MODE_S2B: k_stage_tail<T, KO6, MODE_S2B><<<blocks, TAIL_BLOCK, 0, s>>>(a, v0, twp, nvb); break;
     case MODE_SY: k_stage_tail<T, KO6, MODE_SY><<<blocks, TAIL_BLOCK, 0, s>>>(a, v0, twp, nvb); break;
@@ -194,7 +201,7 @@ int tail_lanes(int width) {
 template <typename T>
 cudaError_t launch_stage_tail(const StageArgs<T> &a, int mode, bool ko6, int v0, int nvb, cudaStream_t s) {
     const int width = a.g.nvs - v0;
-    if (width < 1 || width > 32 || !a.mom_part || nvb < 1) return cudaErrorInvalidValue;
+    if (width < 1 || width > 32 || (!a.mom_part && mode != MODE_RHS) || nvb < 1) return cudaErrorInvalidValue;
     const int twp = tail_lanes(width);
     return ko6 ? launch_tail_ko<T, true>(a, mode, v0, twp, nvb, s) : launch_tail_ko<T, false>(a, mode, v0, twp, nvb, s);
 }

@@ -265,6 +265,25 @@ __device__ __forceinline__ typename VecOf<T>::V vthird_plus(typename VecOf<T>::V
     return vadd(q, vfma(r, third, t));
 }
 
+// one axis's differences of calRHS, taken before any product (adv_axis, ko_axis
+// of physics.cuh): s[-2] - s[2] - 8 (s[-1] - s[1]) and the unit-strength KO sum
+template <typename T, int R, typename V>
+__device__ __forceinline__ V adv_diff(const V (&s)[2 * R + 1]) {
+    using O = VecOf<T>;
+    return vfma(O::splat(-8.0), vsub(s[R - 1], s[R + 1]), vsub(s[R - 2], s[R + 2]));
+}
+template <typename T, int R, typename V>
+__device__ __forceinline__ V ko_sum(const V (&s)[2 * R + 1]) {
+    using O = VecOf<T>;
+    const V t2 = vadd(s[R - 2], s[R + 2]), t1 = vadd(s[R - 1], s[R + 1]);
+    if constexpr (R == 3) {
+        const V t3 = vadd(s[0], s[6]);
+        return vfma(O::splat(-20.0), s[3], vfma(O::splat(15.0), t1, vfma(O::splat(-6.0), t2, t3)));
+    } else {
+        return vfma(O::splat(6.0), s[2], vfma(O::splat(-4.0), t1, t2));
+    }
+}
+
 // statically allocated per-CTA scratch of the march
 struct MarchShared {
     int abort;  // a bounded wait expired
@@ -411,7 +430,7 @@ __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArg
             // flight: box j - NS of a slot was consumed (so had landed) before
             // box j was issued into it -- before the CTA's shared memory is
             // reused or released
-            atomicExch(a.status, NUOSC_TIMEOUT_CODE);
+            if (a.status) atomicExch(a.status, NUOSC_TIMEOUT_CODE);
             for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
                 mbar_wait(smem_u32(&bars[j % NS]), (unsigned)((j / NS) & 1));
         }
@@ -462,14 +481,16 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     const int vp = vb * VB + NP * (lane ^ 16);
     double vx[NP], vy[NP], vz[NP];
     M wo[NP][4], wp[NP][4];
-    V wz[4], wx[4];
+    V wz[4], wx[4], fz, fx;
     {
-        double tz[4][NP], tx[4][NP];
+        double tz[4][NP], tx[4][NP], tfz[NP], tfx[NP];
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             vx[p] = a.q.vx[vc + p];
             vy[p] = a.q.vy[vc + p];
             vz[p] = a.q.vz[vc + p];
+            tfz[p] = vz[p] * a.c.fzs;
+            tfx[p] = vx[p] * a.c.fxs;
             double w4z[4], w4x[4];
             stencil_weights<R>(a.c.kz, __dmul_rn(vz[p], a.c.fzs), w4z);
             stencil_weights<R>(a.c.kx, __dmul_rn(vx[p], a.c.fxs), w4x);
@@ -493,6 +514,8 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) wz[j] = O::make(tz[j]), wx[j] = O::make(tx[j]);
+        fz = O::make(tfz);
+        fx = O::make(tfx);
     }
     const V kz = O::splat(a.c.kz), kx = O::splat(a.c.kx), mu = O::splat(a.c.mu);
     const V kc = O::splat((R == 3 ? -20.0 : 6.0) * (a.c.kz + a.c.kx));  // centre weight of both axes
@@ -506,6 +529,12 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     // to the R..2R-1 others; the move to the next slot is the fma's own
     // destination, so nothing is shifted, and the 2R+1 products of a value are
     // independent of each other.
+    // calRHS keeps the last 2R planes' values themselves (sx[f][row][k] = plane
+    // front - 2R + k) and takes differences first, as the reference does: the
+    // folded weights multiply whole values, whose rounding is that of the state
+    // -- harmless in dt k, which is added to the state, but up to 10 times the
+    // direct kernel's error (2e-6 against 2e-7 in float) when k is the result.
+    constexpr bool RHS = MODE == MODE_RHS;
     V sx[4][RW][2 * R];
     auto tap = [&](int k) -> V {  // weight of a front value in centre (front - R + k)
         return R == 3 ? (k == 0 || k == 6 ? kx : k == 1 ? wx[3] : k == 2 ? wx[2] : k == 3 ? kc : k == 4 ? wx[1] : wx[0])
@@ -533,9 +562,13 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                                    w * g.nvs;
                     const V F = vact ? O::ld(src) : O::zero();
                     auto &q = sx[f][w];
+                    if constexpr (RHS) {
+                        q[R + b] = F;
+                    } else {
 #pragma unroll
-                    for (int k = 0; k + 1 < 2 * R; ++k) q[k] = vfma(tap(k + 1), F, q[k + 1]);
-                    q[2 * R - 1] = vmul(tap(2 * R), F);
+                        for (int k = 0; k + 1 < 2 * R; ++k) q[k] = vfma(tap(k + 1), F, q[k + 1]);
+                        q[2 * R - 1] = vmul(tap(2 * R), F);
+                    }
                 }
         }
     }
@@ -576,17 +609,44 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
             sh.abort = 1;
             break;
         }
-        V y[4][RW];
-        front((const T *)(smem + sf * S::bytes + S::box), y);
-        if (j < R) continue;
-
+        V y[4][RW], cen[4][RW];
+        const T *fb = (const T *)(smem + sf * S::bytes + S::box);
         const unsigned char *sp = smem + sc * S::bytes;
         const T *zb = (const T *)(sp + S::box);
-        V cen[4][RW];
+        if constexpr (RHS) {
 #pragma unroll
-        for (int f = 0; f < 4; ++f)
+            for (int f = 0; f < 4; ++f) {
+                V zs[2 * R + RW];
 #pragma unroll
-            for (int w = 0; w < RW; ++w) cen[f][w] = O::ld(&zb[((r + R + w) * 4 + f) * VB + NP * lane]);
+                for (int k = 0; k < 2 * R + RW; ++k)
+                    if (j >= R) zs[k] = O::ld(&zb[((r + k) * 4 + f) * VB + NP * lane]);
+#pragma unroll
+                for (int w = 0; w < RW; ++w) {
+                    const V F = O::ld(&fb[((r + R + w) * 4 + f) * VB + NP * lane]);
+                    auto &q = sx[f][w];
+                    if (j >= R) {
+                        V z7[2 * R + 1], x7[2 * R + 1];
+#pragma unroll
+                        for (int k = 0; k <= 2 * R; ++k) z7[k] = zs[w + k], x7[k] = k < 2 * R ? q[k < 2 * R ? k : 0] : F;
+                        cen[f][w] = zs[R + w];
+                        y[f][w] = vadd(vfma(fz, adv_diff<T, R>(z7), vmul(fx, adv_diff<T, R>(x7))),
+                                       vfma(kz, ko_sum<T, R>(z7), vmul(kx, ko_sum<T, R>(x7))));
+                    }
+#pragma unroll
+                    for (int k = 0; k + 1 < 2 * R; ++k) q[k] = q[k + 1];
+                    q[2 * R - 1] = F;
+                }
+            }
+        } else {
+            front(fb, y);
+        }
+        if (j < R) continue;
+        if constexpr (!RHS) {
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int w = 0; w < RW; ++w) cen[f][w] = O::ld(&zb[((r + R + w) * 4 + f) * VB + NP * lane]);
+        }
         V pin[4][RW];  // the pointwise input: U (S2, S3) or B (S4)
         if (CF::PU || CF::PA) {
             const T *pb = (const T *)(smem + CF::ring + i % CF::PSM * CF::pbytes);
@@ -632,7 +692,9 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
 #pragma unroll
             for (int f = 0; f < 4; ++f) {
                 const V c = cen[f][w];
-                if (MODE == MODE_S1Y) {
+                if (MODE == MODE_RHS) {
+                    outm[f][w] = kk[f];
+                } else if (MODE == MODE_S1Y) {
                     outm[f][w] = vfma(cY, kk[f], c);  // Y2
                 } else if (MODE == MODE_SY) {
                     outm[f][w] = vfma(cY, kk[f], pin[f][w]);  // Y4
@@ -646,7 +708,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
             }
         }
         if (vact) {
-            T *dp = (MODE == MODE_S4B ? rd<SA>(a.acc_dst) : rd<SA>(a.y_dst)) + hoff + ox;
+            T *dp = (MODE == MODE_S4B || MODE == MODE_RHS ? rd<SA>(a.acc_dst) : rd<SA>(a.y_dst)) + hoff + ox;
 #pragma unroll
             for (int f = 0; f < 4; ++f)
 #pragma unroll
@@ -666,7 +728,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         // follows the loads in program order may overtake them in the pipeline).
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars[NS + sc]));
-        {
+        if constexpr (MODE != MODE_RHS) {
             const bool b4 = lane & 16;
             T ko[4][NP], kp[4][NP];  // the kept row's values: this lane's velocities, the partner's
 #pragma unroll
@@ -721,7 +783,17 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         }
     }
     __syncthreads();
-    return sh.abort != 0;
+    const bool aborted = sh.abort != 0;
+    if constexpr (MODE == MODE_RHS) {  // a caller without a status word sees an incomplete tile as NaN
+        if (aborted && vact)
+            for (int x = xs; x < t.xe; ++x)
+#pragma unroll
+                for (int f = 0; f < 4; ++f)
+#pragma unroll
+                    for (int w = 0; w < RW; ++w)
+                        O::st(a.acc_dst + hoff + f * fs + (long long)x * P + own + w * g.nvs, O::splat(nan("")));
+    }
+    return aborted;
 }
 
 // grid (velocity blocks run by this kernel, z tiles, 2 x x-segments); nvb:
@@ -946,6 +1018,13 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+template <typename T, int TZ>
+cudaError_t launch_rhs_t(const StageArgs<T> &a, bool ko6, XTile t, cudaStream_t s) {
+    if (a.c.pmo != 0.0)
+        return ko6 ? launch_t<T, 3, MODE_RHS, TZ, true, true>(a, t, s) : launch_t<T, 2, MODE_RHS, TZ, true, true>(a, t, s);
+    return ko6 ? launch_t<T, 3, MODE_RHS, TZ, false, true>(a, t, s) : launch_t<T, 2, MODE_RHS, TZ, false, true>(a, t, s);
+}
+
 template <typename T, int R, int TZ, bool VAC, bool M64>
 cudaError_t launch_tm(const StageArgs<T> &a, int mode, XTile t, cudaStream_t s) {
     switch (mode) {
@@ -1133,6 +1212,36 @@ cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t
     return ko6 ? launch_tms<T, 3, 8>(a, mode, t, s) : launch_tms<T, 2, 8>(a, mode, t, s);
 }
 
+// calRHS on the march: 2 state passes (plus the moment pass before it) instead
+// of the direct kernel's 13 or 9 loads per value from L2.  Whole call, moment
+// pass included: 128x128x642 FP64, KO6 1150 -> 567 us (140 of them the moment
+// pass); 250x130x162 FP32, KO4 296 -> 172 us.  The direct kernel stays for nz <
+// 14 and for buffers without 16-byte rows.
+template <typename T>
+bool rhs_xtma_fits(const Geom &g, const void *in, const void *out) {
+    // the tensor maps and the vector accesses need 16-byte aligned rows; a
+    // caller's own buffers may have neither
+    return g.nvs * sizeof(T) % 16 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 &&
+           xtma_fits<T>(g, XTile{g.nz >= 22 ? 16 : 8, 0, vblock<T>()});
+}
+
+template <typename T>
+cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, cudaStream_t s) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int tz = a.g.nz >= 22 ? 16 : 8;
+    const XTile t{tz, xtma_lx<T>(a.g, tz, sms), vblock<T>()};
+    cudaError_t e = tz == 16 ? launch_rhs_t<T, 16>(a, ko6, t, s) : launch_rhs_t<T, 8>(a, ko6, t, s);
+    const int v0 = xtma_tail_v0<T>(a.g);
+    if (e == cudaSuccess && v0 < a.g.nvs)
+        e = launch_stage_tail<T>(a, MODE_RHS, ko6, v0, xtma_num_vblocks<T>(a.g), s);
+    return e;
+}
+
+template bool rhs_xtma_fits<double>(const Geom &, const void *, const void *);
+template bool rhs_xtma_fits<float>(const Geom &, const void *, const void *);
+template cudaError_t launch_rhs_xtma<double>(const StageArgs<double> &, bool, cudaStream_t);
+template cudaError_t launch_rhs_xtma<float>(const StageArgs<float> &, bool, cudaStream_t);
 template bool xtma_supported<double>(const Geom &, XTile);
 template bool xtma_fits<double>(const Geom &, XTile);
 template int xtma_lx<double>(const Geom &, int, int);
