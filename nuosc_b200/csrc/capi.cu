@@ -97,6 +97,7 @@ struct nuosc_handle {
     int kernel = NUOSC_KERNEL_AUTO;
     XTile tile{16, 64, 32};
     bool auto_lx = false;    // tile.lx is xtma_lx's choice for this grid alone
+    int sms = 148;           // SMs of the device
     long long launches = 0;
     bool mom_valid = false;  // d_mom holds the moments of v_stat
     unsigned fault_tx = 0;   // self-test of the TMA kernels' bounded waits (nuosc_selftest_overdeclare_tx)
@@ -338,20 +339,20 @@ int run_stage_xmarch(nuosc_handle *h, bool tma, const XTile &tile, int mode, int
         h->launches++;
     }
     int ps = h->prof_begin(prof_kind(mode));
-    if (tma) {
-        CUDA_TRY(launch_stage_xtma<T>(a, mode, h->ko6, tile, h->stream));
-        const int v0 = xtma_tail_v0<T>(h->g);
-        if (v0 < h->g.nvs) {  // the nearly empty last velocity block
-            CUDA_TRY(launch_stage_tail<T>(a, mode, h->ko6, v0, xtma_num_vblocks<T>(h->g), h->stream));
-            h->launches++;
-        }
+    // (the kernels around a halo exchange are ordered by its copies instead)
+    const bool march = tma && !xtma_all_tail<T>(h->g);
+    const bool early = march && !h->halo && xtma_waves<T>(h->g, tile, h->sms) == 1;
+    if (tma && !march) {
+        CUDA_TRY(launch_stage_tail<T>(a, mode, h->ko6, 0, 1, h->stream));
+    } else if (tma) {
+        CUDA_TRY(launch_stage_xtma<T>(a, mode, h->ko6, tile, early, h->stream));
     } else {
         CUDA_TRY(launch_stage_xmarch<T>(a, mode, h->ko6, tile, h->stream));
     }
     h->prof_end(ps);
     ps = h->prof_begin(5);
     const int nvb = tma ? xtma_num_vblocks<T>(h->g) : xmarch_num_vblocks(h->g, tile);
-    CUDA_TRY(launch_moment_finalize(h->d_part, h->d_mom, h->g, nvb, h->stream));
+    CUDA_TRY(launch_moment_finalize(h->d_part, h->d_mom, h->g, nvb, early, h->stream));
     h->prof_end(ps);
     h->launches += 2;
     h->mom_valid = true;  // d_mom now holds the moments of the register this stage wrote
@@ -883,12 +884,12 @@ int nuosc_create(const nuosc_params *p, nuosc_handle **out) {
     };
     cudaError_t e = cudaSetDevice(h->device);
     if (e != cudaSuccess) return bail(fail(NUOSC_ERR_CUDA, "cudaSetDevice(%d): %s", h->device, cudaGetErrorString(e)));
+    cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
     if (h->tile.lx == 0) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
         // the step falls back to 8-row tiles where 16 rows do not fit
         const int tz = h->tile.tz == 16 && nz < 22 ? 8 : h->tile.tz;
-        h->tile.lx = h->precision == NUOSC_FP64 ? xtma_lx<double>(h->g, tz, sms) : xtma_lx<float>(h->g, tz, sms);
+        h->tile.lx = h->precision == NUOSC_FP64 ? xtma_lx<double>(h->g, tz, h->sms)
+                                                    : xtma_lx<float>(h->g, tz, h->sms);
         h->auto_lx = true;
     }
     e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);

@@ -104,6 +104,29 @@ __host__ __device__ inline long long halo_offset(int F, int p, int nx, int R, lo
     return ((long long)F * 2 * R + hp) * P;
 }
 
+// Programmatic dependent launch, between the march and the moment finalize of a
+// lone solve: each kernel lets the next one be launched from its start, and waits
+// for the one before it (complete, its writes visible) before it touches anything
+// that depends on it.  Both are no-ops in an ordinary launch.
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+#endif
+
 // ---------------------------------------------------------------- launches
 // halt (null by default): a batch member's stop flag; when set, nothing is done
 template <typename T>
@@ -118,6 +141,7 @@ struct XTile {
     int vb;        // velocities per CTA (32)
     int kind = 0;  // preferred x-march kernel from the tile table: 2 cp.async, 3 TMA, 0 either
     int msum = 1;  // FP32 TMA march: moment partials summed in FP64 (1) or in float within a block (0)
+    bool early = false;  // of one launch: it is a single wave (xtma_waves)
 };
 template <typename T>
 bool xmarch_supported(const Geom &g, bool ko6, XTile t);
@@ -133,8 +157,17 @@ bool xtma_supported(const Geom &g, XTile t);
 // x planes per CTA for grid g on a device of `sms` SMs
 template <typename T>
 int xtma_lx(const Geom &g, int tz, int sms);
+// The stage, the tail velocities included; not for grids with xtma_all_tail
 template <typename T>
-cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, cudaStream_t s);
+cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, bool early, cudaStream_t s);
+// waves of CTAs (a tail column included) of the stage's launch on `sms` SMs.  One:
+// all CTAs are resident at once, and the kernel after it may be launched, and wait,
+// while it runs (with more, waiting CTAs would take SMs from the ones still to come)
+template <typename T>
+int xtma_waves(const Geom &g, XTile t, int sms);
+// every velocity fits the tail block: launch_stage_tail runs the stage
+template <typename T>
+bool xtma_all_tail(const Geom &g);
 // calRHS (MODE_RHS: acc_dst = L(in), mom_in = the moments of in) on the TMA
 // march, for grids and buffers it fits
 template <typename T>
@@ -215,7 +248,8 @@ cudaError_t launch_wait_selftest(int *status, unsigned spins, cudaStream_t s);
 // records msg as the calling thread's nuosc_last_error() and returns code (capi.cu)
 int set_last_error(int code, const char *msg);
 int xmarch_num_vblocks(const Geom &g, XTile t);
-cudaError_t launch_moment_finalize(const double *part, double *mom, Geom g, int nvb, cudaStream_t s);
+// early: the march launches around it are single waves (xtma_waves)
+cudaError_t launch_moment_finalize(const double *part, double *mom, Geom g, int nvb, bool early, cudaStream_t s);
 
 template <typename T>
 cudaError_t launch_init(T *reg, const double *G0, const double *G0b, Geom g, int ipt, double eps0,

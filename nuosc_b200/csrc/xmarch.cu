@@ -328,15 +328,16 @@ __global__ void __launch_bounds__(VB *TZ, ctas_per_sm<TZ>()) k_xmarch(StageArgs<
 
 // Sum the partial moments of each cell over velocity blocks and halves in a
 // fixed order: one thread per (cell, moment).
-__global__ void k_moment_finalize(const double *__restrict__ part, double *__restrict__ mom, long long ncell,
-                                  int nvb) {
+__global__ void k_moment_finalize(const double *part, double *mom, long long ncell, int nvb, bool early) {
+    if (early) grid_launch_dependents();
+    grid_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ncell * NMOM) return;
     const long long cell = t / NMOM;
     const int k = (int)(t - cell * NMOM);
     const double *p = part + cell * nvb * 2 * NMOM + k;
     double s = 0.0;
-    for (int b = 0; b < 2 * nvb; ++b) s += p[(long long)b * NMOM];
+    for (int b = 0; b < 2 * nvb; ++b) s += __ldcg(p + (long long)b * NMOM);
     mom[t] = s;
 }
 
@@ -390,10 +391,15 @@ cudaError_t launch_stage_xmarch(const StageArgs<T> &a, int mode, bool ko6, XTile
     return ko6 ? launch_mode<T, 3, 4>(a, mode, t, s) : launch_mode<T, 2, 4>(a, mode, t, s);
 }
 
-cudaError_t launch_moment_finalize(const double *part, double *mom, Geom g, int nvb, cudaStream_t s) {
+cudaError_t launch_moment_finalize(const double *part, double *mom, Geom g, int nvb, bool early, cudaStream_t s) {
     const long long n = g.ncell * NMOM;
-    k_moment_finalize<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(part, mom, g.ncell, nvb);
-    return cudaGetLastError();
+    // the march before and after it fills the SM's shared memory: the same split
+    // spares the SMs a change of configuration twice per stage
+    cudaError_t e = cudaFuncSetAttribute(k_moment_finalize, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(k_moment_finalize, dim3((unsigned)((n + 255) / 256)), 256, 0, s, part, mom, g.ncell, nvb,
+                            early);
 }
 
 namespace {

@@ -53,6 +53,7 @@
 // grid whose CTAs take tiles of many instances from a work-list).
 #include "internal.cuh"
 #include "physics.cuh"
+#include "tail.cuh"
 
 #include <cuda.h>
 
@@ -360,7 +361,7 @@ struct Tile {
 // arrived on the slot's empty barrier, D planes later.
 // fault_tx (the self-test of the bounded waits) over-declares the bytes of box
 // R of the instance's first tile: all its copies land, its phase never completes.
-template <typename T, int R, int MODE, int TZ, bool M64>
+template <typename T, int R, int MODE, int TZ, bool SA>
 __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArgs<T> &a, const Tile &t,
                                              unsigned char *smem, MarchShared &sh) {
     using S = Slot<T, TZ, R>;
@@ -378,6 +379,7 @@ __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArg
     if (lead) {
         const int nx = a.g.nx, nz = a.g.nz, c0 = t.vb * S::VB, c1 = 4 * t.half, nplanes = t.xe - t.xs;
         const bool halo = a.halo != nullptr;
+        if constexpr (!SA) grid_wait();
         for (int j = 0; j < nplanes + R; ++j) {  // centres xs..xe-1 and fronts up to xe-1+R
             const int s = j % NS;
             if (j >= NS && (*(volatile int *)&sh.abort ||
@@ -541,6 +543,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                       : (k == 0 ? wx[3] : k == 1 ? wx[2] : k == 2 ? kc : k == 3 ? wx[1] : wx[0]);
     };
     // the planes left of the segment (periodic, or from a slab's halo buffer)
+    if constexpr (!SA) grid_wait();
     {
         const T *halo = rd<SA>(a.halo);
 #pragma unroll
@@ -796,20 +799,44 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     return aborted;
 }
 
-// grid (velocity blocks run by this kernel, z tiles, 2 x x-segments); nvb:
-// velocity blocks of the moment partials (one more when a tail kernel runs
-// the last block)
+// The tail velocities of a lone solve's launch: block column nvbm, if launched,
+// runs them (first velocity v0, twp lanes per (cell, half)), in launches of up to
+// kTailWaves waves: its CTAs fill the last wave and spare a kernel (us per step:
+// 64x64x162 FP64 208 -> 167, 128x128x162 566 -> 497, 75x150x642 FP32 773 -> 733,
+// 256x256x642 FP32, 5 waves, 4290 -> 3950).  Beyond that a tail CTA, one of few
+// threads per SM and every load a miss, costs more than the kernel that fills the
+// SMs with threads (512x256x642 FP64, 18 waves: 14.7 ms against 13.8).
+constexpr int kTailWaves = 6;
+struct StageTail {
+    int nvbm, v0, twp;
+    bool early;  // one wave: let the next kernel be launched from the start
+};
+
+// grid (velocity blocks run by this kernel + a tail column where there is a tail,
+// z tiles, 2 x x-segments); nvb: velocity blocks of the moment partials
 template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
 __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
-    k_xtma(const __grid_constant__ TmaMaps maps, const StageArgs<T> a, int LX, int nvb) {
+    k_xtma(const __grid_constant__ TmaMaps maps, const StageArgs<T> a, int LX, int nvb, const StageTail f) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ MarchShared sh;
+    constexpr int NC = 32 * (TZ / RW);  // consumer threads
+    if (f.early) grid_launch_dependents();
     const int xs = (blockIdx.z >> 1) * LX;
-    if (xs >= a.g.nx) return;
-    const Tile t{tile_z0(blockIdx.y, gridDim.y, a.g.nz, TZ), (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx), (int)blockIdx.z & 1};
-    if (threadIdx.x >= 32 * (TZ / RW)) {
+    const Tile t{tile_z0(blockIdx.y, gridDim.y, a.g.nz, TZ), (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx),
+                 (int)blockIdx.z & 1};
+    if (blockIdx.x == f.nvbm) {
+        // the tail velocities of the tile's cells: lane l of (plane, row)
+        grid_wait();
+        const int n = (t.xe - t.xs) * TZ * f.twp, step = threads_of(TZ);
+        for (int o = threadIdx.x; o - (int)(threadIdx.x & 31) < n; o += step) {
+            const int l = o & (f.twp - 1), c = o / f.twp;
+            const long long cell = (long long)(xs + c / TZ) * a.g.nz + t.z0 + c % TZ;
+            const int v = f.v0 + l;
+            tail_point<T, R == 3, MODE>(a, cell, t.half, v, o < n && v < a.g.nvs, o < n, f.twp, nvb, l);
+        }
+    } else if (threadIdx.x >= NC) {
         setmaxnreg_dec<RegSplit<TZ>::producer>();
-        xtma_produce<T, R, MODE, TZ, M64>(maps, a, t, smem, sh);
+        xtma_produce<T, R, MODE, TZ, false>(maps, a, t, smem, sh);
     } else {
         setmaxnreg_inc<RegSplit<TZ>::consumer>();
         xtma_consume<T, R, MODE, TZ, VAC, false, M64>(a, t, smem, sh);
@@ -896,7 +923,7 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
             const int w = threadIdx.x - NC;
             if (w < NW) reinterpret_cast<long long *>(&s_a)[w] = reinterpret_cast<const long long *>(&items[lo].a)[w];
             __syncthreads();  // s_a is complete
-            if (xtma_produce<T, R, MODE, TZ, M64>(*s_mp, s_a, s_t, smem, sh)) break;
+            if (xtma_produce<T, R, MODE, TZ, true>(*s_mp, s_a, s_t, smem, sh)) break;
         }
     } else {
         setmaxnreg_inc<RegSplit<TZ>::consumer>();
@@ -979,6 +1006,18 @@ int march_vblocks(const Geom &g) {
     return v0 == g.nvs ? xtma_num_vblocks<T>(g) : v0 / vblock<T>();
 }
 
+}  // namespace
+
+template <typename T>
+int xtma_waves(const Geom &g, XTile t, int sms) {
+    const int cols = march_vblocks<T>(g) + (xtma_tail_v0<T>(g) < g.nvs ? 1 : 0);
+    const long long ctas = 2ll * cols * ((g.nz + t.tz - 1) / t.tz) * ((g.nx + t.lx - 1) / t.lx);
+    const long long slots = (long long)sms * (t.tz == 16 ? 1 : 2);
+    return (int)((ctas + slots - 1) / slots);
+}
+
+namespace {
+
 // the stencil input's boxes, and the TZ-row boxes of the stage's pointwise
 // inputs (U, A) where the stage has them (zeroed maps otherwise)
 template <typename T>
@@ -1005,17 +1044,21 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     TmaMaps maps;
     if (!make_maps<T>(&maps, a, TZ, R)) return cudaErrorInvalidValue;
     const size_t smem = CF::smem;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaError_t e = cudaFuncSetAttribute(k_xtma<T, R, MODE, TZ, VAC, M64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
     const int nseg = (a.g.nx + t.lx - 1) / t.lx;
-    const int nvb = xtma_num_vblocks<T>(a.g), nvbm = march_vblocks<T>(a.g);
-    if (nvbm < 1) return cudaSuccess;  // the tail kernel runs every velocity
+    const int nvb = xtma_num_vblocks<T>(a.g), nvbm = march_vblocks<T>(a.g), v0 = xtma_tail_v0<T>(a.g);
+    const bool tail = v0 < a.g.nvs, column = tail && xtma_waves<T>(a.g, t, sms) <= kTailWaves;
     // velocity blocks fastest: the CTAs resident at once read whole velocity
     // rows of a few z rows (DRAM page locality) rather than one block of many rows
-    dim3 grid(nvbm, (a.g.nz + TZ - 1) / TZ, nseg * 2);
-    k_xtma<T, R, MODE, TZ, VAC, M64><<<grid, threads_of(TZ), smem, s>>>(maps, a, t.lx, nvb);
-    return cudaGetLastError();
+    dim3 grid(nvbm + column, (a.g.nz + TZ - 1) / TZ, nseg * 2);
+    const StageTail f{nvbm, v0, tail_lanes(a.g.nvs - v0), t.early};
+    e = launch_dependent(k_xtma<T, R, MODE, TZ, VAC, M64>, grid, threads_of(TZ), smem, s, maps, a, t.lx, nvb, f);
+    if (e == cudaSuccess && tail && !column) e = launch_stage_tail<T>(a, MODE, R == 3, v0, nvb, s);
+    return e;
 }
 
 template <typename T, int TZ>
@@ -1134,7 +1177,8 @@ bool xtma_supported(const Geom &g, XTile t) {
 template <typename T>
 int xtma_lx(const Geom &g, int tz, int sms) {
     const long long slots = (long long)sms * (tz == 16 ? 1 : 2);
-    const long long per = (long long)((g.nz + tz - 1) / tz) * march_vblocks<T>(g) * 2;  // CTAs per segment
+    const int cols = march_vblocks<T>(g) + (xtma_tail_v0<T>(g) < g.nvs ? 1 : 0);  // (the tail column too)
+    const long long per = (long long)((g.nz + tz - 1) / tz) * cols * 2;  // CTAs per segment
     int best = g.nx;
     double cost = -1.0;
     for (int n = 1; n <= g.nx; ++n) {
@@ -1200,13 +1244,19 @@ int xtma_num_vblocks(const Geom &g) {
 }
 
 template <typename T>
+bool xtma_all_tail(const Geom &g) {
+    return march_vblocks<T>(g) < 1;
+}
+
+template <typename T>
 int xtma_tail_v0(const Geom &g) {
     const int nvb = xtma_num_vblocks<T>(g), last = (nvb - 1) * vblock<T>();
     return 4 * (g.nvs - last) <= vblock<T>() ? last : g.nvs;
 }
 
 template <typename T>
-cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, cudaStream_t s) {
+cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, bool early, cudaStream_t s) {
+    t.early = early;
     if (!a.mom_part || !xtma_fits<T>(a.g, t)) return cudaErrorInvalidValue;
     if (t.tz == 16) return ko6 ? launch_tms<T, 3, 16>(a, mode, t, s) : launch_tms<T, 2, 16>(a, mode, t, s);
     return ko6 ? launch_tms<T, 3, 8>(a, mode, t, s) : launch_tms<T, 2, 8>(a, mode, t, s);
@@ -1231,11 +1281,8 @@ cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, cudaStream_t s) {
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int tz = a.g.nz >= 22 ? 16 : 8;
     const XTile t{tz, xtma_lx<T>(a.g, tz, sms), vblock<T>()};
-    cudaError_t e = tz == 16 ? launch_rhs_t<T, 16>(a, ko6, t, s) : launch_rhs_t<T, 8>(a, ko6, t, s);
-    const int v0 = xtma_tail_v0<T>(a.g);
-    if (e == cudaSuccess && v0 < a.g.nvs)
-        e = launch_stage_tail<T>(a, MODE_RHS, ko6, v0, xtma_num_vblocks<T>(a.g), s);
-    return e;
+    if (xtma_all_tail<T>(a.g)) return launch_stage_tail<T>(a, MODE_RHS, ko6, 0, 1, s);
+    return tz == 16 ? launch_rhs_t<T, 16>(a, ko6, t, s) : launch_rhs_t<T, 8>(a, ko6, t, s);
 }
 
 template bool rhs_xtma_fits<double>(const Geom &, const void *, const void *);
@@ -1245,15 +1292,19 @@ template cudaError_t launch_rhs_xtma<float>(const StageArgs<float> &, bool, cuda
 template bool xtma_supported<double>(const Geom &, XTile);
 template bool xtma_fits<double>(const Geom &, XTile);
 template int xtma_lx<double>(const Geom &, int, int);
+template int xtma_waves<double>(const Geom &, XTile, int);
+template int xtma_waves<float>(const Geom &, XTile, int);
 template int xtma_lx<float>(const Geom &, int, int);
 template bool xtma_fits<float>(const Geom &, XTile);
 template bool xtma_supported<float>(const Geom &, XTile);
 template int xtma_num_vblocks<double>(const Geom &);
 template int xtma_num_vblocks<float>(const Geom &);
 template int xtma_tail_v0<double>(const Geom &);
+template bool xtma_all_tail<double>(const Geom &);
+template bool xtma_all_tail<float>(const Geom &);
 template int xtma_tail_v0<float>(const Geom &);
-template cudaError_t launch_stage_xtma<double>(const StageArgs<double> &, int, bool, XTile, cudaStream_t);
-template cudaError_t launch_stage_xtma<float>(const StageArgs<float> &, int, bool, XTile, cudaStream_t);
+template cudaError_t launch_stage_xtma<double>(const StageArgs<double> &, int, bool, XTile, bool, cudaStream_t);
+template cudaError_t launch_stage_xtma<float>(const StageArgs<float> &, int, bool, XTile, bool, cudaStream_t);
 template size_t xtma_batch_item_bytes<double>();
 template size_t xtma_batch_item_bytes<float>();
 template long long xtma_batch_fill<double>(void *, const StageArgs<double> &, bool, int, int);
