@@ -19,7 +19,7 @@ LIB = os.path.join(HERE, "libnuosc_b200.so")
 OBJ = os.path.join(HERE, "_build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
-              "--expt-relaxed-constexpr", "--split-compile=0", "-I" + os.path.join(ROOT, "include")]
+              "--expt-relaxed-constexpr", "--split-compile=4", "-I" + os.path.join(ROOT, "include")]
 
 
 def nvcc():

@@ -329,15 +329,18 @@ __global__ void __launch_bounds__(VB *TZ, ctas_per_sm<TZ>()) k_xmarch(StageArgs<
 // Sum the partial moments of each cell over velocity blocks and halves in a
 // fixed order: one thread per (cell, moment).
 __global__ void k_moment_finalize(const double *part, double *mom, long long ncell, int nvb, bool early) {
-    if (early) grid_launch_dependents();
-    grid_wait();
+    if (early) {
+        grid_launch_dependents();
+        grid_wait();
+    }
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ncell * NMOM) return;
     const long long cell = t / NMOM;
     const int k = (int)(t - cell * NMOM);
     const double *p = part + cell * nvb * 2 * NMOM + k;
     double s = 0.0;
-    for (int b = 0; b < 2 * nvb; ++b) s += __ldcg(p + (long long)b * NMOM);
+#pragma unroll 4
+    for (int b = 0; b < 2 * nvb; ++b) s += p[(long long)b * NMOM];
     mom[t] = s;
 }
 
@@ -393,13 +396,8 @@ cudaError_t launch_stage_xmarch(const StageArgs<T> &a, int mode, bool ko6, XTile
 
 cudaError_t launch_moment_finalize(const double *part, double *mom, Geom g, int nvb, bool early, cudaStream_t s) {
     const long long n = g.ncell * NMOM;
-    // the march before and after it fills the SM's shared memory: the same split
-    // spares the SMs a change of configuration twice per stage
-    cudaError_t e = cudaFuncSetAttribute(k_moment_finalize, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    return launch_dependent(k_moment_finalize, dim3((unsigned)((n + 255) / 256)), 256, 0, s, part, mom, g.ncell, nvb,
-                            early);
+    return launch_dependent(early, k_moment_finalize, dim3((unsigned)((n + 255) / 256)), 256, 0, s, part, mom, g.ncell,
+                            nvb, early);
 }
 
 namespace {

@@ -363,7 +363,7 @@ struct Tile {
 // R of the instance's first tile: all its copies land, its phase never completes.
 template <typename T, int R, int MODE, int TZ, bool SA>
 __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArgs<T> &a, const Tile &t,
-                                             unsigned char *smem, MarchShared &sh) {
+                                             unsigned char *smem, MarchShared &sh, bool early = false) {
     using S = Slot<T, TZ, R>;
     using CF = MarchCfg<T, R, MODE, TZ>;
     constexpr int NS = CF::NS, ZR = S::ZR;
@@ -379,7 +379,7 @@ __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArg
     if (lead) {
         const int nx = a.g.nx, nz = a.g.nz, c0 = t.vb * S::VB, c1 = 4 * t.half, nplanes = t.xe - t.xs;
         const bool halo = a.halo != nullptr;
-        if constexpr (!SA) grid_wait();
+        if (!SA && early) grid_wait();
         for (int j = 0; j < nplanes + R; ++j) {  // centres xs..xe-1 and fronts up to xe-1+R
             const int s = j % NS;
             if (j >= NS && (*(volatile int *)&sh.abort ||
@@ -444,7 +444,7 @@ __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArg
 // VAC compiles the vacuum term in (it then runs where a.c.pmo != 0).
 template <typename T, int R, int MODE, int TZ, bool VAC, bool SA, bool M64>
 __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &t, unsigned char *smem,
-                                             MarchShared &sh) {
+                                             MarchShared &sh, bool early = false) {
     using S = Slot<T, TZ, R>;
     using CF = MarchCfg<T, R, MODE, TZ>;
     using O = VecOf<T>;
@@ -543,7 +543,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                       : (k == 0 ? wx[3] : k == 1 ? wx[2] : k == 2 ? kc : k == 3 ? wx[1] : wx[0]);
     };
     // the planes left of the segment (periodic, or from a slab's halo buffer)
-    if constexpr (!SA) grid_wait();
+    if (!SA && early) grid_wait();
     {
         const T *halo = rd<SA>(a.halo);
 #pragma unroll
@@ -826,7 +826,7 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
                  (int)blockIdx.z & 1};
     if (blockIdx.x == f.nvbm) {
         // the tail velocities of the tile's cells: lane l of (plane, row)
-        grid_wait();
+        if (f.early) grid_wait();
         const int n = (t.xe - t.xs) * TZ * f.twp, step = threads_of(TZ);
         for (int o = threadIdx.x; o - (int)(threadIdx.x & 31) < n; o += step) {
             const int l = o & (f.twp - 1), c = o / f.twp;
@@ -836,10 +836,10 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
         }
     } else if (threadIdx.x >= NC) {
         setmaxnreg_dec<RegSplit<TZ>::producer>();
-        xtma_produce<T, R, MODE, TZ, false>(maps, a, t, smem, sh);
+        xtma_produce<T, R, MODE, TZ, false>(maps, a, t, smem, sh, f.early);
     } else {
         setmaxnreg_inc<RegSplit<TZ>::consumer>();
-        xtma_consume<T, R, MODE, TZ, VAC, false, M64>(a, t, smem, sh);
+        xtma_consume<T, R, MODE, TZ, VAC, false, M64>(a, t, smem, sh, f.early);
     }
 }
 
@@ -1056,7 +1056,7 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     // rows of a few z rows (DRAM page locality) rather than one block of many rows
     dim3 grid(nvbm + column, (a.g.nz + TZ - 1) / TZ, nseg * 2);
     const StageTail f{nvbm, v0, tail_lanes(a.g.nvs - v0), t.early};
-    e = launch_dependent(k_xtma<T, R, MODE, TZ, VAC, M64>, grid, threads_of(TZ), smem, s, maps, a, t.lx, nvb, f);
+    e = launch_dependent(t.early, k_xtma<T, R, MODE, TZ, VAC, M64>, grid, threads_of(TZ), smem, s, maps, a, t.lx, nvb, f);
     if (e == cudaSuccess && tail && !column) e = launch_stage_tail<T>(a, MODE, R == 3, v0, nvb, s);
     return e;
 }
