@@ -117,7 +117,7 @@ struct nuosc_handle {
     double *d_part = nullptr;  // x-march partial moments
     size_t part_bytes = 0;
     double *d_ana = nullptr;   // analysis partials + final
-    double h_ana[ANA_NQ] = {0};  // analysis read-back
+    double h_ana[ANA_NQ + 1] = {0};  // analysis read-back: sums, status word
     int *d_status = nullptr;
     double *d_stage = nullptr; // host-layout staging
     size_t stage_bytes = 0;
@@ -643,8 +643,8 @@ int upload_spectra(nuosc_handle *h) {
 template <typename T>
 int analysis_raw(nuosc_handle *h, double *q) {
     CUDA_TRY(launch_analysis<T>((const T *)h->reg[0], h->dG0(), h->dG0b(), h->quad().vw, h->g, h->d_ana,
-                                h->d_ana + ANA_BLOCKS * ANA_NQ, h->stream));
-    CUDA_TRY(cudaMemcpyAsync(h->h_ana, h->d_ana + ANA_BLOCKS * ANA_NQ, ANA_NQ * sizeof(double),
+                                h->d_ana + ANA_BLOCKS * ANA_NQ, h->d_status, h->stream));
+    CUDA_TRY(cudaMemcpyAsync(h->h_ana, h->d_ana + ANA_BLOCKS * ANA_NQ, (ANA_NQ + 1) * sizeof(double),
                              cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     memcpy(q, h->h_ana, ANA_NQ * sizeof(double));
@@ -907,7 +907,7 @@ int nuosc_create(const nuosc_params *p, nuosc_handle **out) {
         cudaMemsetAsync(h->reg[r], 0, reg_bytes, h->stream);
     }
     const size_t small = 6 * (size_t)nvs * sizeof(double) + (size_t)h->g.ncell * NMOM * sizeof(double) +
-                         (ANA_BLOCKS + 1) * ANA_NQ * sizeof(double) + 256;
+                         ((ANA_BLOCKS + 1) * ANA_NQ + 1) * sizeof(double) + 256;
     char *blk = nullptr;
     e = dev_alloc((void **)&blk, small, h->device, h->stream);
     if (e != cudaSuccess) return bail(fail(NUOSC_ERR_OOM, "allocating work buffers: %s", cudaGetErrorString(e)));
@@ -1284,9 +1284,10 @@ int nuosc_step_rk4(nuosc_handle *h, int nsteps) {
 
 int nuosc_analysis(nuosc_handle *h, nuosc_diag *o) {
     HANDLE_CHECK(h);
-    if (int rc = check_status(h)) return rc;
     double q[ANA_NQ];
     if (int rc = analysis_dispatch(h, q)) return rc;
+    if (h->h_ana[ANA_NQ] != 0.0)
+        if (int rc = check_status(h)) return rc;
     nuosc_diag d;
     diag_from_sums(h, q, h->phy_time, &d);
     if (o) *o = d;
@@ -1814,7 +1815,7 @@ int batch_step_impl(nuosc_batch *b, int nsteps, int every, nuosc_batch_record *o
                 return fail(NUOSC_ERR_INVALID, "batch_step_stream: more than %d records", max_out);
             double *fin = h->d_ana + ANA_BLOCKS * ANA_NQ;
             CUDA_TRY(launch_analysis<T>((const T *)h->reg[0], h->dG0(), h->dG0b(), h->quad().vw, h->g, h->d_ana, fin,
-                                        b->stream));
+                                        nullptr, b->stream));
             b->kernel_launches += 2;
             if (chk) {  // the stop test on the device; a failed member's later work is skipped
                 CUDA_TRY(launch_halt_check(fin, b->d_halt + i, (int)h->steps_done, b->stream));

@@ -257,12 +257,13 @@ template <typename T>
 cudaError_t launch_init(T *reg, const double *G0, const double *G0b, Geom g, int ipt, double eps0,
                         double sigma, double z0, double dz, uint64_t seed, const double *zprof, int xoff,
                         cudaStream_t s);
-// Analysis partial sums; `part` holds ANA_BLOCKS * ANA_NQ doubles, `out` ANA_NQ.
+// Analysis partial sums; `part` holds ANA_BLOCKS * ANA_NQ doubles, `out` ANA_NQ sums
+// and *status (0 without a status word).
 constexpr int ANA_NQ = 12;
 constexpr int ANA_BLOCKS = 296;
 template <typename T>
 cudaError_t launch_analysis(const T *reg, const double *G0, const double *G0b, const double *vw, Geom g,
-                            double *part, double *out, cudaStream_t s);
+                            double *part, double *out, const int *status, cudaStream_t s);
 template <typename T>
 cudaError_t launch_gather(const T *reg, int field, const int *xidx, int sx, const int *vidx, int sv,
                           const double *G0, const double *G0b, Geom g, double *out, cudaStream_t s);

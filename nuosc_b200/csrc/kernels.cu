@@ -6,10 +6,26 @@
 
 namespace nuosc {
 
+// 16 bytes of consecutive values
+__device__ __forceinline__ void ld16(const double *p, double (&o)[2]) {
+    const double2 t = *reinterpret_cast<const double2 *>(p);
+    o[0] = t.x;
+    o[1] = t.y;
+}
+__device__ __forceinline__ void ld16(const float *p, double (&o)[4]) {
+    const float4 t = *reinterpret_cast<const float4 *>(p);
+    o[0] = t.x;
+    o[1] = t.y;
+    o[2] = t.z;
+    o[3] = t.w;
+}
+
 // ----------------------------------------------------------------------------
 // Velocity moments of one register (nuosc_class.cpp:62-82): one warp per
 // (x,z) cell, lanes stride over v, FP64 accumulation, butterfly warp
-// reduction (fixed order, so the result is deterministic).
+// reduction (fixed order, so the result is deterministic).  HBM-bound:
+// 512x256x642 FP64 0.83 ms, the copy bandwidth (16-byte loads and a
+// reduce-scatter instead of the butterfly were no faster).
 // ----------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) k_moments(const T *__restrict__ in, double *__restrict__ mom, Quad q, Geom g,
@@ -253,41 +269,71 @@ cudaError_t launch_init(T *reg, const double *G0, const double *G0b, Geom g, int
 // 5..7 aM01..aM03, 8 sum w G, 9 sum w Gb, 10 non-finite count, 11 sum w ee^2
 // (with 1 and 8 the advection test's integrals I1, I2, nuosc_ana.cpp:58-61).
 // ----------------------------------------------------------------------------
+//
+// A warp keeps one chunk of velocities (32 lanes x 16 bytes) and strides over the
+// cells, so the spectra, their reciprocals and the weights stay in registers and a
+// point costs its two square roots and the sums, no divide.  Time of the whole
+// analysis() call, one value per load with two divides per point -> this:
+//   64x64x162 FP64 74 -> 37 us, 128x128x642 228 -> 157, 512x256x642 1247 -> 995 (830
+//   of them the state at the copy bandwidth), 256x256x642 FP32 630 -> 569.
 template <typename T>
 __global__ void __launch_bounds__(256) k_analysis(const T *__restrict__ st, const double *__restrict__ G0,
                                                   const double *__restrict__ G0b, const double *__restrict__ vw,
                                                   Geom g, double *__restrict__ part) {
+    constexpr int N = 16 / (int)sizeof(T);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nchunk = (g.nvs + 32 * N - 1) / (32 * N), nwarp = gridDim.x * 8, w = blockIdx.x * 8 + warp;
+    const int chunk = w % nchunk, first = w / nchunk, stride = (nwarp - chunk + nchunk - 1) / nchunk;
+    const int v = chunk * 32 * N + lane * N;
+    double G[N], Gb[N], iG[N], iGb[N], wv[N];
+#pragma unroll
+    for (int p = 0; p < N; ++p) {
+        const bool real = v + p < g.nv;
+        G[p] = real ? G0[v + p] : 1.0;
+        Gb[p] = real ? G0b[v + p] : 1.0;
+        wv[p] = real ? vw[v + p] : 0.0;
+        iG[p] = 1.0 / G[p];
+        iGb[p] = 1.0 / Gb[p];
+    }
     double q[ANA_NQ];
 #pragma unroll
     for (int k = 0; k < ANA_NQ; ++k) q[k] = 0.0;
-    for (long long cell = (long long)blockIdx.x * 8 + warp; cell < g.ncell; cell += (long long)gridDim.x * 8) {
-        const T *row = st + cell * g.nvs;
-        for (int v = lane; v < g.nv; v += 32) {
-            const double ee = row[v], mm = row[v + g.fs], emr = row[v + 2 * g.fs], emi = row[v + 3 * g.fs];
-            const double bee = row[v + 4 * g.fs], bmm = row[v + 5 * g.fs], bemr = row[v + 6 * g.fs],
-                         bemi = row[v + 7 * g.fs];
-            const double G = G0[v], Gb = G0b[v], w = vw[v];
-            const double iG = 1.0 / G, iGb = 1.0 / Gb;
-            const double P1 = 2.0 * emr * iG, P2 = -2.0 * emi * iG, P3 = (ee - mm) * iG;
-            const double P1b = 2.0 * bemr * iGb, P2b = 2.0 * bemi * iGb, P3b = (bee - bmm) * iGb;
-            const double dP = fabs(1.0 - sqrt(P1 * P1 + P2 * P2 + P3 * P3));
-            const double dPb = fabs(1.0 - sqrt(P1b * P1b + P2b * P2b + P3b * P3b));
-            q[0] = fmax(q[0], fmax(dP, dPb));
-            q[1] += w * ee;
-            q[2] += w * bee;
-            q[3] += w * G * dP;
-            q[4] += w * Gb * dPb;
-            q[5] += w * (emr - bemr);
-            q[6] += w * (-emi - bemi);
-            q[7] += w * 0.5 * (ee - mm - bee + bmm);
-            q[8] += w * G;
-            q[9] += w * Gb;
-            q[11] += w * ee * ee;
-            const double chk = ee + mm + emr + emi + bee + bmm + bemr + bemi;
-            if (!isfinite(chk)) q[10] += 1.0;
+    long long cells = 0;
+    if (v < g.nv)
+        for (long long cell = first; cell < g.ncell; cell += stride, ++cells) {
+            const T *row = st + cell * g.nvs + v;
+            double f[NF][N];
+#pragma unroll
+            for (int k = 0; k < NF; ++k) ld16(row + k * g.fs, f[k]);
+#pragma unroll
+            for (int p = 0; p < N; ++p) {
+                if (p > 0 && v + p >= g.nv) break;  // padding of the last vector
+                const double ee = f[0][p], mm = f[1][p], emr = f[2][p], emi = f[3][p];
+                const double bee = f[4][p], bmm = f[5][p], bemr = f[6][p], bemi = f[7][p];
+                const double P1 = 2.0 * emr * iG[p], P2 = -2.0 * emi * iG[p], P3 = (ee - mm) * iG[p];
+                const double P1b = 2.0 * bemr * iGb[p], P2b = 2.0 * bemi * iGb[p], P3b = (bee - bmm) * iGb[p];
+                const double dP = fabs(1.0 - sqrt(P1 * P1 + P2 * P2 + P3 * P3));
+                const double dPb = fabs(1.0 - sqrt(P1b * P1b + P2b * P2b + P3b * P3b));
+                const double w = wv[p];
+                q[0] = fmax(q[0], fmax(dP, dPb));
+                q[1] += w * ee;
+                q[2] += w * bee;
+                q[3] += w * G[p] * dP;
+                q[4] += w * Gb[p] * dPb;
+                q[5] += w * (emr - bemr);
+                q[6] += w * (-emi - bemi);
+                q[7] += w * 0.5 * (ee - mm - bee + bmm);
+                q[11] += w * ee * ee;
+                const double chk = ee + mm + emr + emi + bee + bmm + bemr + bemi;
+                if (!isfinite(chk)) q[10] += 1.0;
+            }
         }
-    }
+#pragma unroll
+    for (int p = 0; p < N; ++p)
+        if (v + p < g.nv) {  // the same in every cell
+            q[8] += (double)cells * (wv[p] * G[p]);
+            q[9] += (double)cells * (wv[p] * Gb[p]);
+        }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         q[0] = fmax(q[0], __shfl_xor_sync(0xffffffffu, q[0], off));
@@ -307,19 +353,33 @@ __global__ void __launch_bounds__(256) k_analysis(const T *__restrict__ st, cons
     }
 }
 
-__global__ void k_analysis_final(const double *__restrict__ part, int nblocks, double *__restrict__ out) {
-    const int k = threadIdx.x;
-    if (k >= ANA_NQ) return;
-    double r = part[k];
-    for (int b = 1; b < nblocks; ++b) r = (k == 0) ? fmax(r, part[b * ANA_NQ + k]) : r + part[b * ANA_NQ + k];
-    out[k] = r;
+// One warp per quantity: lane l sums blocks l, l + 32, ..., then the lanes in a
+// fixed order (one thread per quantity walked 296 partials, about 40 us).  *status,
+// the handle's word of expired waits, goes out with the sums, so that one copy
+// brings both to the host.
+__global__ void k_analysis_final(const double *__restrict__ part, int nblocks, double *__restrict__ out,
+                                 const int *__restrict__ status) {
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double r = 0.0;  // (quantity 0, a maximum, is not negative)
+#pragma unroll 5
+    for (int b = lane; b < nblocks; b += 32) {
+        const double p = part[b * ANA_NQ + k];
+        r = k == 0 ? fmax(r, p) : r + p;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const double p = __shfl_xor_sync(0xffffffffu, r, off);
+        r = k == 0 ? fmax(r, p) : r + p;
+    }
+    if (lane == 0) out[k] = r;
+    if (threadIdx.x == 0) out[ANA_NQ] = status ? (double)*status : 0.0;
 }
 
 template <typename T>
 cudaError_t launch_analysis(const T *reg, const double *G0, const double *G0b, const double *vw, Geom g,
-                            double *part, double *out, cudaStream_t s) {
+                            double *part, double *out, const int *status, cudaStream_t s) {
     k_analysis<T><<<ANA_BLOCKS, 256, 0, s>>>(reg, G0, G0b, vw, g, part);
-    k_analysis_final<<<1, 32, 0, s>>>(part, ANA_BLOCKS, out);
+    k_analysis_final<<<1, 32 * ANA_NQ, 0, s>>>(part, ANA_BLOCKS, out, status);
     return cudaGetLastError();
 }
 
@@ -482,7 +542,7 @@ cudaError_t launch_renormalize(T *reg, const double *G0, const double *G0b, Geom
     template cudaError_t launch_init<T>(T *, const double *, const double *, Geom, int, double, double, double, \
                                         double, uint64_t, const double *, int, cudaStream_t);                 \
     template cudaError_t launch_analysis<T>(const T *, const double *, const double *, const double *, Geom,   \
-                                            double *, double *, cudaStream_t);                                \
+                                            double *, double *, const int *, cudaStream_t);                   \
     template cudaError_t launch_gather<T>(const T *, int, const int *, int, const int *, int, const double *,  \
                                           const double *, Geom, double *, cudaStream_t);                      \
     template cudaError_t launch_import<T>(T *, const double *, Geom, int, int, int, cudaStream_t);            \
