@@ -474,6 +474,28 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     const unsigned fs32 = (unsigned)fs, P32 = (unsigned)P, own32 = (unsigned)own;
     __syncthreads();  // the barriers are initialised
 
+    // the R planes left of the segment (periodic, or from a slab's halo buffer),
+    // loaded ahead of the constants so that their latencies overlap
+    V pre[R][4][RW];
+    if (!SA && early) grid_wait();
+    {
+        const T *halo = rd<SA>(a.halo);
+#pragma unroll
+        for (int b = 0; b < R; ++b) {
+            const int pl = xs - R + b;
+            const bool hal = halo != nullptr && pl < 0;
+            const long long o = (long long)wrap_index(pl, g.nx) * P + own;
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int w = 0; w < RW; ++w) {
+                    const T *src = (hal ? halo + halo_offset(4 * half + f, pl, g.nx, R, P) + own : in + f * fs + o) +
+                                   w * g.nvs;
+                    pre[b][f][w] = vact ? O::ld(src) : O::zero();
+                }
+        }
+    }
+
     // per-velocity constants, in registers.  Lane-permuted moment weights: slot s
     // of a lane holds weight s ^ wq (weights w, w vx, w vy, w vz), wq = lane bits
     // 3..2, the order the moment reduce-scatter needs; of this lane's
@@ -542,39 +564,25 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         return R == 3 ? (k == 0 || k == 6 ? kx : k == 1 ? wx[3] : k == 2 ? wx[2] : k == 3 ? kc : k == 4 ? wx[1] : wx[0])
                       : (k == 0 ? wx[3] : k == 1 ? wx[2] : k == 2 ? kc : k == 3 ? wx[1] : wx[0]);
     };
-    // the planes left of the segment (periodic, or from a slab's halo buffer)
-    if (!SA && early) grid_wait();
-    {
-        const T *halo = rd<SA>(a.halo);
 #pragma unroll
-        for (int f = 0; f < 4; ++f)
+    for (int f = 0; f < 4; ++f)
 #pragma unroll
-            for (int w = 0; w < RW; ++w)
+        for (int w = 0; w < RW; ++w) {
+            auto &q = sx[f][w];
 #pragma unroll
-                for (int k = 0; k < 2 * R; ++k) sx[f][w][k] = O::zero();
+            for (int k = 0; k < 2 * R; ++k) q[k] = O::zero();
 #pragma unroll
-        for (int b = 0; b < R; ++b) {
-            const int pl = xs - R + b;
-            const bool hal = halo != nullptr && pl < 0;
-            const long long o = (long long)wrap_index(pl, g.nx) * P + own;
+            for (int b = 0; b < R; ++b) {
+                const V F = pre[b][f][w];
+                if constexpr (RHS) {
+                    q[R + b] = F;
+                } else {
 #pragma unroll
-            for (int f = 0; f < 4; ++f)
-#pragma unroll
-                for (int w = 0; w < RW; ++w) {
-                    const T *src = (hal ? halo + halo_offset(4 * half + f, pl, g.nx, R, P) + own : in + f * fs + o) +
-                                   w * g.nvs;
-                    const V F = vact ? O::ld(src) : O::zero();
-                    auto &q = sx[f][w];
-                    if constexpr (RHS) {
-                        q[R + b] = F;
-                    } else {
-#pragma unroll
-                        for (int k = 0; k + 1 < 2 * R; ++k) q[k] = vfma(tap(k + 1), F, q[k + 1]);
-                        q[2 * R - 1] = vmul(tap(2 * R), F);
-                    }
+                    for (int k = 0; k + 1 < 2 * R; ++k) q[k] = vfma(tap(k + 1), F, q[k + 1]);
+                    q[2 * R - 1] = vmul(tap(2 * R), F);
                 }
+            }
         }
-    }
     // front j of the march: box j's values enter the x sums and, with their z
     // sums, the centre sum of their own plane; y = the completed stencil sums
     // of centre j - R
