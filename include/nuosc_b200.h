@@ -68,10 +68,10 @@ extern "C" {
 #define NUOSC_LAYOUT_GHOSTED 1 /* the reference's array: [(i+gx)*(nz+2gz)+j+gz]*nv+v (CartGrid.h:91) */
 
 /* stage-kernel selection (nuosc_set_kernel) */
-#define NUOSC_KERNEL_AUTO 0   /* the TMA x-march kernel when the geometry allows, else the cp.async one */
+#define NUOSC_KERNEL_AUTO 0   /* the TMA x-march kernel (any nz >= 14), else the cp.async one */
 #define NUOSC_KERNEL_DIRECT 1 /* one thread per (cell, velocity), separate moment pass */
 #define NUOSC_KERNEL_XMARCH 2 /* cp.async-staged x-march with fused moments (any geometry) */
-#define NUOSC_KERNEL_XTMA 3   /* TMA-fed x-march with mbarrier ring, fused moments (nz % tz == 0) */
+#define NUOSC_KERNEL_XTMA 3   /* TMA-fed x-march with mbarrier ring, fused moments; asked for by name: nz % tz == 0 */
 
 typedef struct nuosc_handle nuosc_handle;
 
@@ -130,8 +130,9 @@ int nuosc_set_renorm(nuosc_handle *h, int renorm);
 /* stage-kernel choice (NUOSC_KERNEL_*); no counterpart in the reference */
 int nuosc_set_kernel(nuosc_handle *h, int kind);
 /* x-march tile: tz z-rows per CTA (4, 8 or 16) and lx x-planes marched per CTA.
- * The default comes from the autotuner's table (tiles.txt beside the
- * library, keyed on velocity count and precision).  No reference counterpart. */
+ * The default comes from the autotuner's table (tiles.txt beside the library,
+ * keyed on velocity count and precision); where that leaves lx open, from the
+ * grid and the device's SM count.  No reference counterpart. */
 int nuosc_set_tile(nuosc_handle *h, int tz, int lx);
 int nuosc_get_tile(const nuosc_handle *h, int *tz, int *lx);
 /* How the FP32 TMA kernel sums the velocity-moment partials of a 64-velocity

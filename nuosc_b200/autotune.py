@@ -14,8 +14,7 @@ error is within MSUM_TOL.  With --write the choice goes to
 nuosc_b200/tiles.txt ("nv precision tz lx kernel msum" per line), which the
 library reads when a handle is created (lx 0 there, as in the table that comes
 with the library, leaves the segment length to a rule on the grid).  The direct
-kernel is timed too, for
-reference.  Results are printed as one JSON line.
+kernel is timed too, for reference.  Results are printed as one JSON line.
 
 The velocity block of the TMA kernel is not a tuning dimension: it is one
 warp's lanes (32 velocities in FP64, 64 in FP32 with two per lane), since the

@@ -1,20 +1,21 @@
 // tail.cu -- the last, nearly empty velocity block of an x-march stage.
 //
 // The TMA x-march kernel runs 32 (FP64) or 64 (FP32) velocities per CTA, one
-// or two per lane.  When nv leaves only a few velocities in the last block
+// 8-byte value per lane.  When nv leaves only a few velocities in the last block
 // (642 = 20 x 32 + 2 in FP64, 644 = 10 x 64 + 4 in FP32), a CTA for that
 // block would issue a full block's instructions for a handful of active
 // lanes -- up to a tenth of the stage's issue slots.  Those tail velocities
 // are computed here instead, one thread per (cell, tail velocity, flavour
-// half) with 4 fields, the stencil read through the read-only cache (the
+// half) with 4 fields (tail.cuh), the stencil read with plain loads (the
 // tail columns of a few planes stay in L2), the same fused RK epilogue, and
 // the velocity-moment partials of the written state summed over the tail
 // lanes of the (cell, half) into the last block's slots of the partial
 // array, so the fixed-order moment_finalize is unchanged.
 //
-// A solve stepped alone runs its tail in CTAs of the march launch itself
-// (xtma.cu); the kernels here run the tails of a batch, and a solve whose
-// velocities all fit the tail (12 velocities in FP32).
+// A solve stepped alone in launches of up to 6 waves runs its tail in CTAs of
+// the march launch itself (xtma.cu); the kernels here run the tails of larger
+// launches and of a batch, and a solve whose velocities all fit the tail (12
+// velocities in FP32).
 #include "internal.cuh"
 #include "tail.cuh"
 

@@ -33,10 +33,10 @@
 // the status word, stops marching and, before returning, waits (again
 // bounded) for the copies it issued.  nz need not be a multiple of TZ (tile_z0).
 //
-// What bounds it, measured on a 512 x 256 x 642 FP64 grid (KO6): S1 2.8 ms (2
-// state passes, 3.9 TB/s) is held by instruction latency at 8 consumer warps
+// What bounds it, measured on a 512 x 256 x 642 FP64 grid (KO6): S1 2.6 ms (2
+// state passes, 4.1 TB/s) is held by instruction latency at 8 consumer warps
 // per SM (two per scheduler: the partial sums alone take 96 registers); S2 4.5,
-// S3 3.1, S4 3.2 ms run at 4.8-5.2 TB/s of the 6.5 a plain copy reaches.  The
+// S3 3.1, S4 3.1 ms run at 4.8-5.2 TB/s of the 6.5 a plain copy reaches.  The
 // form before -- 16 warps of one point per thread, a 7-deep register queue in x
 // shifted every plane, weights read from shared memory, plain loads of the
 // pointwise inputs, warp 0 issuing the copies -- took 3.9 / 5.0 / 4.5 / 4.6 ms:
@@ -1019,7 +1019,8 @@ int march_vblocks(const Geom &g) {
 template <typename T>
 int xtma_waves(const Geom &g, XTile t, int sms) {
     const int cols = march_vblocks<T>(g) + (xtma_tail_v0<T>(g) < g.nvs ? 1 : 0);
-    const long long ctas = 2ll * cols * ((g.nz + t.tz - 1) / t.tz) * ((g.nx + t.lx - 1) / t.lx);
+    const int lx = t.lx < g.nx ? t.lx : g.nx;
+    const long long ctas = 2ll * cols * ((g.nz + t.tz - 1) / t.tz) * ((g.nx + lx - 1) / lx);
     const long long slots = (long long)sms * (t.tz == 16 ? 1 : 2);
     return (int)((ctas + slots - 1) / slots);
 }
@@ -1057,6 +1058,7 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(k_xtma<T, R, MODE, TZ, VAC, M64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
+    if (t.lx > a.g.nx) t.lx = a.g.nx;  // (one segment)
     const int nseg = (a.g.nx + t.lx - 1) / t.lx;
     const int nvb = xtma_num_vblocks<T>(a.g), nvbm = march_vblocks<T>(a.g), v0 = xtma_tail_v0<T>(a.g);
     const bool tail = v0 < a.g.nvs, column = tail && xtma_waves<T>(a.g, t, sms) <= kTailWaves;
@@ -1190,6 +1192,8 @@ int xtma_lx(const Geom &g, int tz, int sms) {
     int best = g.nx;
     double cost = -1.0;
     for (int n = 1; n <= g.nx; ++n) {
+        // n or more segments (at least n / 2 once rounded) cannot cost less than this
+        if (cost >= 0.0 && (double)per * (n / 2) / (double)slots * 11.0 > cost) break;
         const int lx = (g.nx + n - 1) / n, nseg = (g.nx + lx - 1) / lx;
         const double c = (double)((per * nseg + slots - 1) / slots) * (lx + 10);
         if (cost < 0.0 || c < 0.98 * cost) {
