@@ -57,6 +57,7 @@
 
 #include <cuda.h>
 
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 #include <utility>
@@ -1182,16 +1183,26 @@ bool xtma_supported(const Geom &g, XTile t) {
 // best of a sweep over lx in brackets): 32x32x42 lx 2: 53 [53], 16: 109, 32:
 // 174; 64x64x162 lx 22: 208 [208], 32: 238, 64: 371; 128x128x162 lx 43: 570
 // [566], 32: 636, 64: 749; 128x128x642 lx 64: 1817 [1817], 128: 2015;
-// 100x90x162 lx 50: 344 [344], 34: 426, 100: 525; from 512x256x642 on every lx
-// from 40 to 256 is within 2 %.
+// 100x90x162 lx 50: 344 [344], 34: 426, 100: 525.
+//
+// Where many whole waves make all counts cost the same, two limits stand.  CTAs
+// drift apart along a long march, and neighbouring velocity blocks then no longer
+// read a DRAM page together: at most 192 planes (ms per step: 256x256x642 FP64 lx
+// 256: 7.5, 128: 7.3, 86: 7.1; 1024x256x642 FP64 lx 1024: 32.6, 512: 29.1, 64 to
+// 256: 28.7 to 29.0).  And a segment spans at most 2 GiB of a register, as the
+// pages in use at a time grow with it: 1024x1024x642 FP64 (172 GB) lx 1024: 128,
+// 256: 122, 128: 122, 64: 117.5, 48: 116.3 (the choice), 32: 118, 24: 120.6; FP32
+// lx 1024: 64.8, 96 (the choice): 63.2, 48: 64.1.
 template <typename T>
 int xtma_lx(const Geom &g, int tz, int sms) {
     const long long slots = (long long)sms * (tz == 16 ? 1 : 2);
     const int cols = march_vblocks<T>(g) + (xtma_tail_v0<T>(g) < g.nvs ? 1 : 0);  // (the tail column too)
     const long long per = (long long)((g.nz + tz - 1) / tz) * cols * 2;  // CTAs per segment
-    int best = g.nx;
+    const double span = (double)g.nx * g.nz * g.nvs * 8 * sizeof(T) / (1ll << 31);  // 2 GiB pieces of a register
+    int first = (g.nx + 191) / 192, best = 1;
+    if (span > first) first = span < g.nx ? (int)ceil(span) : g.nx;
     double cost = -1.0;
-    for (int n = 1; n <= g.nx; ++n) {
+    for (int n = first; n <= g.nx; ++n) {
         // n or more segments (at least n / 2 once rounded) cannot cost less than this
         if (cost >= 0.0 && (double)per * (n / 2) / (double)slots * 11.0 > cost) break;
         const int lx = (g.nx + n - 1) / n, nseg = (g.nx + lx - 1) / lx;
