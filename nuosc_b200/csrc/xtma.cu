@@ -1192,7 +1192,8 @@ bool xtma_supported(const Geom &g, XTile t) {
 // 256: 28.7 to 29.0).  And a segment spans at most 2 GiB of a register, as the
 // pages in use at a time grow with it: 1024x1024x642 FP64 (172 GB) lx 1024: 128,
 // 256: 122, 128: 122, 64: 117.5, 48: 116.3 (the choice), 32: 118, 24: 120.6; FP32
-// lx 1024: 64.8, 96 (the choice): 63.2, 48: 64.1.
+// lx 1024: 64.8, 94 to 96 (the choice): 63.2, 48: 64.1; 512x512x642 FP32 lx 512:
+// 16.6, 171: 15.1.  (128x1024x642 FP64 pays 1 %: lx 128 14.15, 43 14.35.)
 template <typename T>
 int xtma_lx(const Geom &g, int tz, int sms) {
     const long long slots = (long long)sms * (tz == 16 ? 1 : 2);
