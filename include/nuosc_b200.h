@@ -300,6 +300,11 @@ int nuosc_selftest_wait_timeout(int device, unsigned spins, double *ms);
  * state is undefined until it is set again.  0 switches the test off. */
 int nuosc_selftest_overdeclare_tx(nuosc_handle *h, unsigned extra_bytes);
 
+/* Self-test of the TMA kernels' z tiles (host arithmetic only; no reference
+ * counterpart): the first row of tile `tile` of the tz-row tiles (8 or 16) of
+ * nz rows; NUOSC_ERR_INVALID where there is no such tile. */
+int nuosc_selftest_z_tile(int nz, int tz, int tile, int *z0);
+
 /* Per-kernel timing with CUDA events on the handle's stream (no counterpart
  * in the reference, which prints wall time per step, nuosc.cpp:222-235).
  * Kinds: 0 stage S1, 1 stage S2 (and S3 on the direct and cp.async paths),

@@ -104,6 +104,21 @@ __host__ __device__ inline long long halo_offset(int F, int p, int nx, int R, lo
     return ((long long)F * 2 * R + hp) * P;
 }
 
+// The z tiles of a march: ceil(nz / tz) tiles of tz rows (at least two: nz >= tz +
+// 6).  Where tz does not divide nz they are spread evenly and overlap.
+// Neighbouring tiles are at least 3 >= R rows apart, so only the first and the
+// last tile's box crosses the periodic end and the box pieces are those of an
+// exact division.  Tile t starts at row t (nz - tz) / (tiles - 1), formed as t q +
+// t rem / (tiles - 1) with the host's q and rem: the product in one piece leaves 32
+// bits from nz = 131,080 (8 rows) or 185,377 (16 rows), while t and rem are below
+// 65,535, the largest grid's y extent, and their product below 2^32.
+struct ZTiles {
+    unsigned n, q, rem;
+    ZTiles(int nz, int tz)
+        : n((unsigned)((nz + tz - 1) / tz)), q((unsigned)(nz - tz) / (n - 1)), rem((unsigned)(nz - tz) % (n - 1)) {}
+    __host__ __device__ int row(unsigned t) const { return (int)(t * q + t * rem / (n - 1)); }
+};
+
 // Programmatic dependent launch, between the march and the moment finalize of a
 // lone solve whose march is a single wave (`early`): each kernel lets the next one
 // be launched from its start, and waits for the one before it (complete, its

@@ -31,7 +31,7 @@
 //     stop test) has its tiles skipped.
 // All mbarrier waits are bounded: on expiry the kernel records the timeout in
 // the status word, stops marching and, before returning, waits (again
-// bounded) for the copies it issued.  nz need not be a multiple of TZ (tile_z0).
+// bounded) for the copies it issued.  nz need not be a multiple of TZ (ZTiles).
 //
 // What bounds it, measured on a 512 x 256 x 642 FP64 grid (KO6): S1 2.6 ms (2
 // state passes, 4.1 TB/s) is held by instruction latency at 8 consumer warps
@@ -332,14 +332,6 @@ __device__ __forceinline__ P rd(const P &x) {
     if constexpr (V) return *(const volatile P *)&x;
     else return x;
 }
-
-// First row of z tile zt of ntz.  Where TZ does not divide nz, the ntz =
-// ceil(nz / TZ) tiles are spread evenly and overlap: rows of two tiles are
-// computed twice, to the same bits (no stage writes what it reads).  With nz >=
-// TZ + 6 neighbouring tiles are at least 3 >= R rows apart, so only the first
-// and the last tile's box crosses the periodic end and the box pieces are those
-// of an exact division.
-__device__ __forceinline__ int tile_z0(int zt, int ntz, int nz, int tz) { return zt * (nz - tz) / (ntz - 1); }
 
 // One tile of work: z rows z0..z0+TZ-1, velocity block vb (of nvb), x planes
 // xs..xe-1, flavour half `half`
@@ -825,13 +817,14 @@ struct StageTail {
 // z tiles, 2 x x-segments); nvb: velocity blocks of the moment partials
 template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
 __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
-    k_xtma(const __grid_constant__ TmaMaps maps, const StageArgs<T> a, int LX, int nvb, const StageTail f) {
+    k_xtma(const __grid_constant__ TmaMaps maps, const StageArgs<T> a, const ZTiles zt, int LX, int nvb,
+           const StageTail f) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ MarchShared sh;
     constexpr int NC = 32 * (TZ / RW);  // consumer threads
     if (f.early) grid_launch_dependents();
     const int xs = (blockIdx.z >> 1) * LX;
-    const Tile t{tile_z0(blockIdx.y, gridDim.y, a.g.nz, TZ), (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx),
+    const Tile t{zt.row(blockIdx.y), (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx),
                  (int)blockIdx.z & 1};
     if (blockIdx.x == f.nvbm) {
         // the tail velocities of the tile's cells: lane l of (plane, row)
@@ -1065,9 +1058,11 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     const bool tail = v0 < a.g.nvs, column = tail && xtma_waves<T>(a.g, t, sms) <= kTailWaves;
     // velocity blocks fastest: the CTAs resident at once read whole velocity
     // rows of a few z rows (DRAM page locality) rather than one block of many rows
-    dim3 grid(nvbm + column, (a.g.nz + TZ - 1) / TZ, nseg * 2);
+    const ZTiles zt(a.g.nz, TZ);
+    dim3 grid(nvbm + column, zt.n, nseg * 2);
     const StageTail f{nvbm, v0, tail_lanes(a.g.nvs - v0), t.early};
-    e = launch_dependent(t.early, k_xtma<T, R, MODE, TZ, VAC, M64>, grid, threads_of(TZ), smem, s, maps, a, t.lx, nvb, f);
+    e = launch_dependent(t.early, k_xtma<T, R, MODE, TZ, VAC, M64>, grid, threads_of(TZ), smem, s, maps, a, zt, t.lx,
+                         nvb, f);
     if (e == cudaSuccess && tail && !column) e = launch_stage_tail<T>(a, MODE, R == 3, v0, nvb, s);
     return e;
 }
