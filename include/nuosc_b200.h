@@ -302,8 +302,9 @@ int nuosc_selftest_overdeclare_tx(nuosc_handle *h, unsigned extra_bytes);
 
 /* Self-test of the TMA kernels' z tiles (host arithmetic only; no reference
  * counterpart): the first row of tile `tile` of the tz-row tiles (8 or 16) of
- * nz rows; NUOSC_ERR_INVALID where there is no such tile. */
-int nuosc_selftest_z_tile(int nz, int tz, int tile, int *z0);
+ * nz rows, and how many rows from there on the tile before stores (0 where tz
+ * divides nz); NUOSC_ERR_INVALID where there is no such tile. */
+int nuosc_selftest_z_tile(int nz, int tz, int tile, int *z0, int *skip);
 
 /* Per-kernel timing with CUDA events on the handle's stream (no counterpart
  * in the reference, which prints wall time per step, nuosc.cpp:222-235).

@@ -133,7 +133,7 @@ _SIGS = {
     "nuosc_release_cached_memory": [_I],
     "nuosc_selftest_wait_timeout": [_I, C.c_uint, C.POINTER(C.c_double)],
     "nuosc_selftest_overdeclare_tx": [_P, C.c_uint],
-    "nuosc_selftest_z_tile": [_I, _I, _I, _IP],
+    "nuosc_selftest_z_tile": [_I, _I, _I, _IP, _IP],
 }
 PROF_KINDS = ["stage_s1", "stage_s2", "stage_s4", "calrhs", "moments", "moment_finalize", "stage_s3"]
 

@@ -2024,11 +2024,12 @@ int nuosc_selftest_wait_timeout(int device, unsigned spins, double *ms) {
     return fail(NUOSC_ERR_TIMEOUT, "selftest: the bounded wait expired after %u polls (%.3f ms)", spins, el);
 }
 
-int nuosc_selftest_z_tile(int nz, int tz, int tile, int *z0) {
+int nuosc_selftest_z_tile(int nz, int tz, int tile, int *z0, int *skip) {
     if ((tz != 8 && tz != 16) || nz < tz + 6 || nz >= 1 << 30 || tile < 0 || tile >= (nz + tz - 1) / tz ||
         (nz + tz - 1) / tz > 65535)
         return fail(NUOSC_ERR_INVALID, "z_tile: tile %d of %d-row tiles of %d rows", tile, tz, nz);
     if (z0) *z0 = ZTiles(nz, tz).row((unsigned)tile);
+    if (skip) *skip = ZTiles(nz, tz).shared_rows((unsigned)tile, tz);
     return NUOSC_OK;
 }
 

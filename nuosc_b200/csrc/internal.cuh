@@ -117,6 +117,11 @@ struct ZTiles {
     ZTiles(int nz, int tz)
         : n((unsigned)((nz + tz - 1) / tz)), q((unsigned)(nz - tz) / (n - 1)), rem((unsigned)(nz - tz) % (n - 1)) {}
     __host__ __device__ int row(unsigned t) const { return (int)(t * q + t * rem / (n - 1)); }
+    // rows at the start of tile t that tile t - 1 has too: they are tile t - 1's to
+    // store, so that every row is stored by one tile (q is tz where tz divides nz)
+    __host__ __device__ int shared_rows(unsigned t, int tz) const {
+        return t > 0 && q != (unsigned)tz ? tz - (row(t) - row(t - 1)) : 0;
+    }
 };
 
 // Programmatic dependent launch, between the march and the moment finalize of a

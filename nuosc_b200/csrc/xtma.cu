@@ -130,6 +130,7 @@ struct VecOf<double> {
     static __device__ __forceinline__ V ld(const double *p) { return *p; }
     static __device__ __forceinline__ void st(double *p, V a) { *p = a; }
     static __device__ __forceinline__ V zero() { return 0.0; }
+    static __device__ __forceinline__ unsigned long long bits(V a) { return __double_as_longlong(a); }
 };
 template <>
 struct VecOf<float> {
@@ -144,6 +145,7 @@ struct VecOf<float> {
     }
     static __device__ __forceinline__ void st(float *p, V a) { *reinterpret_cast<unsigned long long *>(p) = a.v; }
     static __device__ __forceinline__ V zero() { return f2{0ull}; }
+    static __device__ __forceinline__ unsigned long long bits(V a) { return a.v; }
 };
 
 struct __align__(64) TmaMaps {
@@ -288,7 +290,8 @@ __device__ __forceinline__ V ko_sum(const V (&s)[2 * R + 1]) {
 
 // statically allocated per-CTA scratch of the march
 struct MarchShared {
-    int abort;  // a bounded wait expired
+    unsigned long long sink;  // a lane's values of a row that is not the tile's to store
+    int abort;                // a bounded wait expired
 };
 
 template <typename T, int TZ>
@@ -334,9 +337,10 @@ __device__ __forceinline__ P rd(const P &x) {
 }
 
 // One tile of work: z rows z0..z0+TZ-1, velocity block vb (of nvb), x planes
-// xs..xe-1, flavour half `half`
+// xs..xe-1, flavour half `half`.  The first `skip` rows are the tile before's
+// (ZTiles): nothing of them is stored here.
 struct Tile {
-    int z0, vb, nvb, xs, xe, half;
+    int z0, vb, nvb, xs, xe, half, skip;
 };
 
 // The march of one tile of the instance (maps, a): every thread of the CTA calls
@@ -434,8 +438,9 @@ __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArg
     return aborted;
 }
 
-// VAC compiles the vacuum term in (it then runs where a.c.pmo != 0).
-template <typename T, int R, int MODE, int TZ, bool VAC, bool SA, bool M64>
+// VAC compiles the vacuum term in (it then runs where a.c.pmo != 0), RAG the rows
+// that are the tile before's (grids that TZ does not divide).
+template <typename T, int R, int MODE, int TZ, bool VAC, bool SA, bool M64, bool RAG>
 __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &t, unsigned char *smem,
                                              MarchShared &sh, bool early = false) {
     using S = Slot<T, TZ, R>;
@@ -465,7 +470,21 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     // all fit (xtma_supported requires 3 fs < 2^32); only the half's own
     // offset, hoff, needs 64 bits
     const unsigned fs32 = (unsigned)fs, P32 = (unsigned)P, own32 = (unsigned)own;
+    // RAG: where both rows are the tile before's the warp only takes its part in the
+    // ring; where the first is (keep0 false) the second alone is stored
+    const bool keep0 = !RAG || t.skip <= r;
     __syncthreads();  // the barriers are initialised
+    if (RAG && t.skip >= r + RW) {
+        for (int j = 0; j < nboxes; ++j) {
+            if (!mbar_wait(smem_u32(&bars[j % NS]), (unsigned)((j / NS) & 1)) || *(volatile int *)&sh.abort) {
+                sh.abort = 1;
+                break;
+            }
+            if (j >= R && lane == 0) mbar_arrive(smem_u32(&bars[NS + (j - R) % NS]));
+        }
+        __syncthreads();
+        return sh.abort != 0;
+    }
 
     // the R planes left of the segment (periodic, or from a slab's halo buffer),
     // loaded ahead of the constants so that their latencies overlap
@@ -711,7 +730,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                 }
             }
         }
-        if (vact) {
+        if (vact && keep0) {
             T *dp = (MODE == MODE_S4B || MODE == MODE_RHS ? rd<SA>(a.acc_dst) : rd<SA>(a.y_dst)) + hoff + ox;
 #pragma unroll
             for (int f = 0; f < 4; ++f)
@@ -725,11 +744,22 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                     for (int w = 0; w < RW; ++w) O::st(bp + f * fs32 + w * g.nvs, outb[f][w]);
             }
         }
+        if (RAG && !keep0) {
+            const long long o = hoff + ox + g.nvs;
+            T *dp = (MODE == MODE_S4B || MODE == MODE_RHS ? a.acc_dst : a.y_dst) + o;
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                if (vact) O::st(dp + f * fs, outm[f][1]);
+                if (MODE == MODE_S2B && vact) O::st(a.acc_dst + o + f * fs, outb[f][1]);
+                if (lane == 0) *(volatile unsigned long long *)&sh.sink = O::bits(outm[f][0]);
+            }
+        }
         // The centre use is the box's last (a right-halo box has none: its slot is
         // not filled again).  The arrive comes after the stores: they need every
         // value this plane read from shared memory, so no such read can still be
         // under way when the producer refills the slots (an arrive that only
-        // follows the loads in program order may overtake them in the pipeline).
+        // follows the loads in program order may overtake them in the pipeline); the
+        // values of a row that is not stored are written to sh.sink instead.
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars[NS + sc]));
         if constexpr (MODE != MODE_RHS) {
@@ -777,7 +807,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
             const M k1 = acc[1][0] + __shfl_xor_sync(0xffffffffu, acc[1][0], 2);
             M kk = (!b1 && b0) ? k1 : k0;
             kk += __shfl_xor_sync(0xffffffffu, (b1 || b0) ? k0 : k1, 1);
-            if (!(b1 && b0)) {  // lane holds moment 4c + wq of its kept row
+            if (!(b1 && b0) && (b4 || keep0)) {  // lane holds moment 4c + wq of its kept row
                 const int c = b1 ? 2 : (int)b0;
                 const double v = (double)kk;
                 const unsigned cell = (unsigned)x * (unsigned)rd<SA>(a.g.nz) + (unsigned)(zr + (b4 ? 1 : 0));
@@ -795,7 +825,8 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                 for (int f = 0; f < 4; ++f)
 #pragma unroll
                     for (int w = 0; w < RW; ++w)
-                        O::st(a.acc_dst + hoff + f * fs + (long long)x * P + own + w * g.nvs, O::splat(nan("")));
+                        if (w > 0 || keep0)
+                            O::st(a.acc_dst + hoff + f * fs + (long long)x * P + own + w * g.nvs, O::splat(nan("")));
     }
     return aborted;
 }
@@ -815,7 +846,7 @@ struct StageTail {
 
 // grid (velocity blocks run by this kernel + a tail column where there is a tail,
 // z tiles, 2 x x-segments); nvb: velocity blocks of the moment partials
-template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
+template <typename T, int R, int MODE, int TZ, bool VAC, bool M64, bool RAG>
 __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
     k_xtma(const __grid_constant__ TmaMaps maps, const StageArgs<T> a, const ZTiles zt, int LX, int nvb,
            const StageTail f) {
@@ -825,7 +856,7 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
     if (f.early) grid_launch_dependents();
     const int xs = (blockIdx.z >> 1) * LX;
     const Tile t{zt.row(blockIdx.y), (int)blockIdx.x, nvb, xs, min(xs + LX, a.g.nx),
-                 (int)blockIdx.z & 1};
+                 (int)blockIdx.z & 1, RAG ? zt.shared_rows(blockIdx.y, TZ) : 0};
     if (blockIdx.x == f.nvbm) {
         // the tail velocities of the tile's cells: lane l of (plane, row)
         if (f.early) grid_wait();
@@ -834,14 +865,15 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
             const int l = o & (f.twp - 1), c = o / f.twp;
             const long long cell = (long long)(xs + c / TZ) * a.g.nz + t.z0 + c % TZ;
             const int v = f.v0 + l;
-            tail_point<T, R == 3, MODE>(a, cell, t.half, v, o < n && v < a.g.nvs, o < n, f.twp, nvb, l);
+            const bool own = o < n && (!RAG || c % TZ >= t.skip);
+            tail_point<T, R == 3, MODE>(a, cell, t.half, v, own && v < a.g.nvs, own, f.twp, nvb, l);
         }
     } else if (threadIdx.x >= NC) {
         setmaxnreg_dec<RegSplit<TZ>::producer>();
         xtma_produce<T, R, MODE, TZ, false>(maps, a, t, smem, sh, f.early);
     } else {
         setmaxnreg_inc<RegSplit<TZ>::consumer>();
-        xtma_consume<T, R, MODE, TZ, VAC, false, M64>(a, t, smem, sh, f.early);
+        xtma_consume<T, R, MODE, TZ, VAC, false, M64, RAG>(a, t, smem, sh, f.early);
     }
 }
 
@@ -907,6 +939,7 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
                     s_t.xs = (loc >> 1) * e.lx;
                     s_t.xe = min(s_t.xs + e.lx, e.a.g.nx);
                     s_t.nvb = e.nvb;
+                    s_t.skip = 0;
                     s_mp = &e.maps;
                     // this thread issues every TMA load of the tile; the maps were written
                     // through the generic proxy (a host copy when the work-list was built)
@@ -936,7 +969,7 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
             if (lo == -1) break;
             if (lo == -2) continue;
             __syncthreads();
-            if (xtma_consume<T, R, MODE, TZ, VAC, true, M64>(s_a, s_t, smem, sh)) break;
+            if (xtma_consume<T, R, MODE, TZ, VAC, true, M64, false>(s_a, s_t, smem, sh)) break;
         }
     }
 }
@@ -1049,8 +1082,9 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     const size_t smem = CF::smem;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(k_xtma<T, R, MODE, TZ, VAC, M64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    const ZTiles zt(a.g.nz, TZ);
+    const auto kern = a.g.nz % TZ ? k_xtma<T, R, MODE, TZ, VAC, M64, true> : k_xtma<T, R, MODE, TZ, VAC, M64, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if (t.lx > a.g.nx) t.lx = a.g.nx;  // (one segment)
     const int nseg = (a.g.nx + t.lx - 1) / t.lx;
@@ -1058,11 +1092,9 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     const bool tail = v0 < a.g.nvs, column = tail && xtma_waves<T>(a.g, t, sms) <= kTailWaves;
     // velocity blocks fastest: the CTAs resident at once read whole velocity
     // rows of a few z rows (DRAM page locality) rather than one block of many rows
-    const ZTiles zt(a.g.nz, TZ);
     dim3 grid(nvbm + column, zt.n, nseg * 2);
     const StageTail f{nvbm, v0, tail_lanes(a.g.nvs - v0), t.early};
-    e = launch_dependent(t.early, k_xtma<T, R, MODE, TZ, VAC, M64>, grid, threads_of(TZ), smem, s, maps, a, zt, t.lx,
-                         nvb, f);
+    e = launch_dependent(t.early, kern, grid, threads_of(TZ), smem, s, maps, a, zt, t.lx, nvb, f);
     if (e == cudaSuccess && tail && !column) e = launch_stage_tail<T>(a, MODE, R == 3, v0, nvb, s);
     return e;
 }

@@ -1,5 +1,6 @@
 """The z tiles of the TMA kernels, on the host arithmetic that the launches use
-(no GPU): every tile lies inside the grid, whatever its size."""
+(no GPU): every tile lies inside the grid, whatever its size, and every row is
+stored by one tile."""
 import ctypes as C
 
 import pytest
@@ -8,9 +9,9 @@ from nuosc_b200 import _lib
 
 
 def z_tile(lib, nz, tz, tile):
-    z0 = C.c_int()
-    _lib.check(lib.nuosc_selftest_z_tile(nz, tz, tile, C.byref(z0)))
-    return z0.value
+    z0, skip = C.c_int(), C.c_int()
+    _lib.check(lib.nuosc_selftest_z_tile(nz, tz, tile, C.byref(z0), C.byref(skip)))
+    return z0.value, skip.value
 
 
 @pytest.fixture(scope="module")
@@ -32,15 +33,17 @@ def test_starts(lib, tz):
         if -(-nz // tz) > 65535:
             continue
         n = -(-nz // tz)
-        starts = rows_of(lib, nz, tz)
-        assert starts == [t * (nz - tz) // (n - 1) for t in range(n)]
+        starts, skip = zip(*rows_of(lib, nz, tz))
+        assert list(starts) == [t * (nz - tz) // (n - 1) for t in range(n)]
         assert starts[0] == 0 and starts[-1] == nz - tz
         if nz % tz == 0:
-            assert starts == list(range(0, nz, tz))
+            assert list(starts) == list(range(0, nz, tz)) and not any(skip)
         # no gap, and at least as far apart as the widest halo (3 rows)
         assert all(3 <= b - a <= tz for a, b in zip(starts, starts[1:]))
+        # the rows that the tiles store follow each other and are all of the grid's
+        assert [a + k for a, k in zip(starts, skip)] == [0] + [a + tz for a in starts[:-1]]
 
 
 def test_no_such_tile(lib):
     for nz, tz, tile in ((90, 12, 0), (21, 16, 0), (90, 16, 6), (90, 16, -1), (65535 * 16 + 1, 16, 0)):
-        assert lib.nuosc_selftest_z_tile(nz, tz, tile, None) == _lib.ERR_INVALID
+        assert lib.nuosc_selftest_z_tile(nz, tz, tile, None, None) == _lib.ERR_INVALID
