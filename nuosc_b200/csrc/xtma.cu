@@ -23,7 +23,8 @@
 //     products of a value do not depend on each other;
 //   * moment partials (FP64 products and sums; FP32 state may sum in float
 //     within the block, stored as double): a warp's half-warps exchange values
-//     so that each keeps one row, each lane forms the 12 products (3
+//     so that the lower one keeps the grid's even row and the upper one the odd
+//     one (no sum depends on the tile that a row falls into), each lane forms the 12 products (3
 //     combinations x 4 weights, the weights in a lane-permuted order set once
 //     per tile) of its own and its partner's velocities, and the half-warp
 //     reduce-scatters them with 12 shuffle-adds;
@@ -763,7 +764,10 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bars[NS + sc]));
         if constexpr (MODE != MODE_RHS) {
-            const bool b4 = lane & 16;
+            // the half-warp that keeps a row decides whose product is rounded first
+            // (its own velocity's), so the lower one keeps the row that is even in
+            // the grid: RAG tiles may start at an odd one
+            const bool b4 = RAG ? ((lane >> 4) ^ z0) & 1 : lane & 16;
             T ko[4][NP], kp[4][NP];  // the kept row's values: this lane's velocities, the partner's
 #pragma unroll
             for (int f = 0; f < 4; ++f) {

@@ -1,7 +1,8 @@
 """Grids that no tile height divides are repeatable bit for bit: every row of
 the state and of the moment partials is stored by one tile, so no result
 depends on which of two overlapping tiles comes last, and a solve continued
-from a checkpoint equals the uninterrupted one."""
+from a checkpoint equals the uninterrupted one.  Nor does a result depend on the
+tile's height or on where in a tile a row lies."""
 import numpy as np
 import pytest
 
@@ -53,3 +54,17 @@ def test_repeatable(nb, nz, precision, ghost, nn, tmp_path):
     b.step_rk4(7)
     assert np.array_equal(bits(b), ref)
     b.close()
+
+
+# 8- and 16-row tiles put a row at an odd place in one tile and at an even one in
+# the other; segments of one and of many planes
+@pytest.mark.parametrize("nz", [22, 33, 49, 90, 150])
+@pytest.mark.parametrize("precision,ghost,nn", [(0, 3, 4), (0, 2, 3), (1, 3, 3), (1, 2, 4)])
+def test_tile_independent(nb, nz, precision, ghost, nn):
+    ref = None
+    for tile in ((16, 128), (8, 128), (16, 3), (8, 5)):
+        s = make(nb, 24, nz, nn, precision, ghost, tile)
+        s.step_rk4(5)
+        ref = bits(s) if ref is None else ref
+        assert np.array_equal(bits(s), ref), tile
+        s.close()
