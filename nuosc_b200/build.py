@@ -6,6 +6,7 @@ nvcc cross-compiles without a GPU.  Every .cu/.cpp under csrc/ is compiled
 with -gencode arch=compute_100a,code=sm_100a and linked into one shared
 library exporting the C ABI of include/nuosc_b200.h.
 """
+import concurrent.futures
 import glob
 import os
 import shutil
@@ -17,9 +18,10 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnuosc_b200.so")
 OBJ = os.path.join(HERE, "_build")
+PARTS = {"xtma.cu": 11}  # sources compiled in parts, -DNUOSC_PART=0 ... n-1
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
-              "--expt-relaxed-constexpr", "--split-compile=4", "-I" + os.path.join(ROOT, "include")]
+              "--expt-relaxed-constexpr", "-I" + os.path.join(ROOT, "include")]
 
 
 def nvcc():
@@ -43,21 +45,22 @@ def _stale(obj, src, deps):
 def build(verbose=False, jobs=8, extra=()):
     os.makedirs(OBJ, exist_ok=True)
     headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + \
-        glob.glob(os.path.join(ROOT, "include", "*.h"))
+        glob.glob(os.path.join(ROOT, "include", "*.h")) + [os.path.abspath(__file__)]  # (its flags)
     cc = nvcc()
-    procs, objs = [], []
+    jobs_list, objs = [], []
     for src in sources():
-        obj = os.path.join(OBJ, os.path.basename(src) + ".o")
-        objs.append(obj)
-        if not _stale(obj, src, headers):
-            continue
-        cmd = [cc] + ARCH + NVCC_FLAGS + list(extra) + ["-x", "cu", "-c", src, "-o", obj]
-        if verbose:
-            print(" ".join(cmd))
-        procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
-        if len(procs) >= jobs:
-            _drain(procs)
-    _drain(procs)
+        name = os.path.basename(src)
+        for part in range(PARTS.get(name, 1)):
+            whole = name not in PARTS
+            obj = os.path.join(OBJ, name + (".o" if whole else ".%d.o" % part))
+            objs.append(obj)
+            if _stale(obj, src, headers):
+                define = [] if whole else ["-DNUOSC_PART=%d" % part]
+                jobs_list.append(
+                    (obj, [cc] + ARCH + NVCC_FLAGS + list(extra) + define + ["-x", "cu", "-c", src, "-o", obj]))
+    jobs_list.sort(key=lambda j: "xtma" not in j[0])  # the longest first
+    with concurrent.futures.ThreadPoolExecutor(jobs) as pool:
+        _check(pool.map(lambda j: _compile(*j, verbose), jobs_list))
     if not os.path.exists(LIB) or any(os.path.getmtime(o) > os.path.getmtime(LIB) for o in objs):
         cmd = [cc] + ARCH + ["-shared", "-cudart", "static", "-o", LIB] + objs
         if verbose:
@@ -85,15 +88,25 @@ def build_driver(verbose=False):
     return exe
 
 
-def _drain(procs):
+def _compile(obj, cmd, verbose):
+    if verbose:
+        print(" ".join(cmd))
+    # to another name first: an interrupted build leaves no object that looks up to date
+    tmp = obj + ".tmp"
+    r = subprocess.run(cmd[:-1] + [tmp], stdout=subprocess.PIPE, stderr=subprocess.STDOUT)
+    if r.returncode == 0:
+        os.replace(tmp, obj)
+    return obj, r
+
+
+def _check(results):
     errs = []
-    for src, p in procs:
-        out, _ = p.communicate()
-        if p.returncode != 0:
-            errs.append("%s:\n%s" % (src, out.decode(errors="replace")))
-        elif out.strip():
-            sys.stderr.write(out.decode(errors="replace"))
-    procs.clear()
+    for obj, r in results:
+        text = r.stdout.decode(errors="replace")
+        if r.returncode != 0:
+            errs.append("%s:\n%s" % (obj, text))
+        elif text.strip():
+            sys.stderr.write(text)
     if errs:
         raise RuntimeError("nvcc failed\n" + "\n".join(errs))
 

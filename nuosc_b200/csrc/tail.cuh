@@ -7,6 +7,18 @@
 
 namespace nuosc {
 
+// *p; issued in program order, so that all of a field's loads are in flight at once
+__device__ __forceinline__ double ld_now(const double *p) {
+    double r;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float ld_now(const float *p) {
+    float r;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
+    return r;
+}
+
 // One (cell, velocity, flavour half) of the tail; every lane of the warp
 // calls it (the moment reduction shuffles across the twp lanes of a cell and
 // half), act says whether the lane holds a real point.  twp: lanes per
@@ -23,27 +35,25 @@ __device__ __forceinline__ void tail_point(const StageArgs<T> &a, const long lon
 #pragma unroll
     for (int k = 0; k < NMOM; ++k) mom[k] = 0.0;
     if (act) {
-        const int i = (int)(cell / g.nz), j = (int)(cell - (long long)i * g.nz);
+        const int i = (int)((unsigned)cell / (unsigned)g.nz), j = (int)((unsigned)cell - (unsigned)i * (unsigned)g.nz);
         constexpr int R = KO6 ? 3 : 2;
         const long long hoff = (long long)half * 4 * g.fs;
-        const long long P = (long long)g.nz * g.nvs;
-        // x neighbours: field-0 pointer of this half and field stride per
-        // offset -- inside the register (periodic), or a slab's halo buffer
-        long long oz[7];
-        const T *xp[7];
+        const long long P = (long long)g.nz * g.nvs, col = (long long)j * g.nvs + v, ctr = (long long)i * P + col;
+        const T *in = a.in + hoff;
+        const T *halo = a.halo ? a.halo + (long long)half * 8 * R * P : nullptr;
+        // neighbours: field-0 pointers of this half and the x ones' field stride --
+        // inside the register (periodic), or a slab's halo buffer
+        const T *zp[7], *xp[7];
         long long xfs[7];
 #pragma unroll
         for (int k = -3; k <= 3; ++k) {
             const int kk = (k < -R || k > R) ? 0 : k;
-            oz[k + 3] = ((long long)i * g.nz + wrap_index(j + kk, g.nz)) * g.nvs + v;
-            const int pl = i + kk;
-            if (a.halo && (pl < 0 || pl >= g.nx)) {
-                xp[k + 3] = a.halo + halo_offset(4 * half, pl, g.nx, R, P) + (long long)j * g.nvs + v;
-                xfs[k + 3] = 2 * R * P;
-            } else {
-                xp[k + 3] = a.in + hoff + ((long long)wrap_index(pl, g.nx) * g.nz + j) * g.nvs + v;
-                xfs[k + 3] = g.fs;
-            }
+            const int jz = j + kk, pl = i + kk;  // (nz, nx > 3: one wrap at most)
+            zp[k + 3] = in + (ctr + (long long)(jz < 0 ? kk + g.nz : jz >= g.nz ? kk - g.nz : kk) * g.nvs);
+            const bool out = pl < 0 || pl >= g.nx, hal = out && halo != nullptr;
+            const int px = pl < 0 ? (hal ? pl + R : pl + g.nx) : pl >= g.nx ? (hal ? pl - g.nx + R : pl - g.nx) : pl;
+            xp[k + 3] = (hal ? halo : in) + ((long long)px * P + col);
+            xfs[k + 3] = hal ? 2 * R * P : g.fs;
         }
         const double vxd = a.q.vx[v], vyd = a.q.vy[v], vzd = a.q.vz[v], wd = a.q.vw[v];
         const T fx = T(vxd * a.c.fxs), fz = T(vzd * a.c.fzs);
@@ -53,20 +63,20 @@ __device__ __forceinline__ void tail_point(const StageArgs<T> &a, const long lon
         T c4[4], a4[4], k4[4];
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
-            const T *F = a.in + hoff + f * g.fs;
             T zs[7], xs[7];
 #pragma unroll
             for (int k = 0; k < 7; ++k) {
-                zs[k] = F[oz[k]];
-                xs[k] = xp[k][f * xfs[k]];
+                const bool used = k >= 3 - R && k <= 3 + R;
+                zs[k] = used ? ld_now(zp[k] + f * g.fs) : T(0);
+                xs[k] = used && k != 3 ? ld_now(xp[k] + f * xfs[k]) : T(0);
             }
-            c4[f] = zs[3];
+            xs[3] = c4[f] = zs[3];
             a4[f] = adv_axis(zs, fz) + adv_axis(xs, fx);
             k4[f] = ko_axis<T, KO6>(zs, kz) + ko_axis<T, KO6>(xs, kx);
         }
         T kv[4];
         commutator_half(c4, ia, ib, ie, a.c, kv, a4, k4);
-        const long long o = oz[3] + hoff;
+        const long long o = ctr + hoff;
         const T cA = T(a.cA), cY = T(a.cY);
         T outm[4];  // the written state whose moments the next stage needs
 #pragma unroll

@@ -4,7 +4,7 @@
 // x one flavour half and marches along x:
 //   * a producer warpgroup (one issuing lane) loads, for every x plane the CTA
 //     touches, the plane's [TZ+2R rows][4 fields][velocities] box with one TMA
-//     tensor load (cp.async.bulk.tensor.4d; 2-3 boxes where the periodic z wrap
+//     tensor load (cp.async.bulk.tensor.4d; two where the periodic z wrap
 //     cuts it), the TZ cells' moments with a bulk copy, and the stage's
 //     pointwise input (U in S2 and S3, B in S4; none in S1) of the plane that
 //     the box completes, into shared-memory rings whose completion is tracked
@@ -49,6 +49,15 @@
 // (a late warp starves all), issue by the last warp to release a slot 3.3.
 // FP32 (same grid): 2.2 / 2.8 / 2.4 / 2.5 -> 1.7 / 2.2 / 1.8 / 1.8 ms.
 //
+// The file is compiled in parts (NUOSC_PART, build.py), each with its share of the
+// kernels: the whole in one piece takes 7 minutes.  (nvcc's --split-compile halves
+// that, but one source then gave one of two codes by chance, 5 to 8 % apart, small
+// grids up to 18 %.)  What the compiler decided in the one or the other way is
+// written out: a loop for the fronts that complete no centre, loads in program
+// order, no branch on what is the same in every plane.  Against the better of the
+// two codes (geometric mean over 16 to 512 cells a side, 12 to 642 velocities):
+// steps FP64 1.04, FP32 1.11, calRHS 1.07 and 1.09, batches 1.01 to 1.13.
+//
 // The march of one tile is a device function shared by two kernels: k_xtma
 // (one tile per CTA, one instance per launch) and k_xtma_batch (a persistent
 // grid whose CTAs take tiles of many instances from a work-list).
@@ -62,6 +71,11 @@
 #include <cstring>
 #include <type_traits>
 #include <utility>
+
+#ifndef NUOSC_PART
+#error "compiled once per part: -DNUOSC_PART=0 ... 10"
+#endif
+#pragma nv_diag_suppress 177  // each part leaves some functions unused
 
 namespace nuosc {
 
@@ -120,6 +134,14 @@ __device__ __forceinline__ f2 vmul(f2 a, f2 b) {
 __device__ __forceinline__ f2 vsub(f2 a, f2 b) { return vfma(b, pack(-1.f, -1.f), a); }
 __device__ __forceinline__ f2 vneg(f2 a) { return f2{a.v ^ 0x8000000080000000ull}; }
 
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Loads and predicated stores of a value, in program order (volatile) and without a
+// branch: conditions that are the same in every plane (a lane past the last
+// velocity, a row that is not the tile's) must not become control flow, which the
+// compiler hoists out of the march by copying the loop, and worse code.
+//   ldg: *p from global memory where `on`, else 0;  lds: from shared memory
+//   st_if: to global memory where `on`
 template <typename T>
 struct VecOf;
 template <>
@@ -128,8 +150,26 @@ struct VecOf<double> {
     static __device__ __forceinline__ V splat(double x) { return x; }
     static __device__ __forceinline__ V make(const double (&x)[1]) { return x[0]; }
     static __device__ __forceinline__ void get(V a, double (&x)[1]) { x[0] = a; }
-    static __device__ __forceinline__ V ld(const double *p) { return *p; }
-    static __device__ __forceinline__ void st(double *p, V a) { *p = a; }
+    static __device__ __forceinline__ V ldg(const double *p, int on) {
+        V r;
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n mov.f64 %0, 0d0000000000000000;\n @p ld.global.f64 %0, "
+            "[%1];\n}\n"
+            : "=d"(r)
+            : "l"(p), "r"(on)
+            : "memory");
+        return r;
+    }
+    static __device__ __forceinline__ V lds(const double *p) {
+        V r;
+        asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(r) : "r"(smem_u32(p)));
+        return r;
+    }
+    static __device__ __forceinline__ void st_if(double *p, V a, int on) {
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p st.global.f64 [%0], %1;\n}\n" ::"l"(p), "d"(a),
+                     "r"(on)
+                     : "memory");
+    }
     static __device__ __forceinline__ V zero() { return 0.0; }
     static __device__ __forceinline__ unsigned long long bits(V a) { return __double_as_longlong(a); }
 };
@@ -141,10 +181,25 @@ struct VecOf<float> {
     static __device__ __forceinline__ void get(V a, float (&x)[2]) {
         asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(a.v));
     }
-    static __device__ __forceinline__ V ld(const float *p) {
-        return f2{*reinterpret_cast<const unsigned long long *>(p)};
+    static __device__ __forceinline__ V ldg(const float *p, int on) {
+        V r;
+        asm volatile(
+            "{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n mov.b64 %0, 0;\n @p ld.global.b64 %0, [%1];\n}\n"
+            : "=l"(r.v)
+            : "l"(p), "r"(on)
+            : "memory");
+        return r;
     }
-    static __device__ __forceinline__ void st(float *p, V a) { *reinterpret_cast<unsigned long long *>(p) = a.v; }
+    static __device__ __forceinline__ V lds(const float *p) {
+        V r;
+        asm volatile("ld.shared.b64 %0, [%1];\n" : "=l"(r.v) : "r"(smem_u32(p)));
+        return r;
+    }
+    static __device__ __forceinline__ void st_if(float *p, V a, int on) {
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p st.global.b64 [%0], %1;\n}\n" ::"l"(p), "l"(a.v),
+                     "r"(on)
+                     : "memory");
+    }
     static __device__ __forceinline__ V zero() { return f2{0ull}; }
     static __device__ __forceinline__ unsigned long long bits(V a) { return a.v; }
 };
@@ -152,15 +207,14 @@ struct VecOf<float> {
 struct __align__(64) TmaMaps {
     CUtensorMap zr;   // box of TZ+2R rows (plane box with both halos)
     CUtensorMap tzr;  // TZ+R rows (a box cut by the wrap)
-    CUtensorMap tz;   // TZ rows (middle piece of a box wrapped at both ends)
     CUtensorMap r;    // R rows (wrapped halo)
     CUtensorMap pu;   // TZ rows of the stage's U register (pointwise input)
     CUtensorMap pa;   // TZ rows of the final stage's B input (acc_src; pointwise)
-    // the same four box shapes over a slab's halo buffer (planes right of the slab)
-    CUtensorMap hzr, htzr, htz, hr;
+    // the same three box shapes over a slab's halo buffer (planes right of the slab),
+    // kHalo maps further on
+    CUtensorMap hzr, htzr, hr;
+    static constexpr int kHalo = 5;
 };
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
@@ -181,6 +235,7 @@ __device__ __forceinline__ void setmaxnreg_dec() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(N));
 }
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigned spins = kWaitSpins) {
+#pragma unroll 1
     for (unsigned it = 0; it < spins; ++it) {
         unsigned ok;
         asm volatile(
@@ -206,6 +261,10 @@ __device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap *map
         "%5}], [%6];\n" ::"r"(dst),
         "l"((unsigned long long)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
         : "memory");
+}
+__device__ __forceinline__ void sink_if(unsigned dst, unsigned long long x, int on) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p st.shared.b64 [%0], %1;\n}\n" ::"r"(dst), "l"(x), "r"(on)
+                 : "memory");
 }
 __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
@@ -377,47 +436,45 @@ __device__ __forceinline__ bool xtma_produce(const TmaMaps &maps, const StageArg
     if (lead) {
         const int nx = a.g.nx, nz = a.g.nz, c0 = t.vb * S::VB, c1 = 4 * t.half, nplanes = t.xe - t.xs;
         const bool halo = a.halo != nullptr;
+        // the box in z, the same for every plane: one piece, or two where the periodic
+        // wrap cuts it (the first tile's after R rows, the last one's before the last R)
+        const int cut = t.z0 == 0 ? R : t.z0 + TZ == nz ? TZ + R : ZR;
+        const int za = t.z0 == 0 ? nz - R : t.z0 - R;
+        const CUtensorMap *piece1 = cut == ZR ? &maps.zr : cut == R ? &maps.r : &maps.tzr;
+        const CUtensorMap *piece2 = cut == R ? &maps.tzr : &maps.r;
+        const double *mom = a.mom_in + (long long)t.z0 * NMOM;
+        const unsigned fault_tx = t.z0 == 0 && t.vb == 0 && t.xs == 0 && t.half == 0 ? a.fault_tx : 0u;
         if (!SA && early) grid_wait();
+        int s = 0, ps = 0;       // slots of box j and of the pointwise rows of plane j - R
+        unsigned refills = 0;    // times slot s has been filled
+#pragma unroll 1
         for (int j = 0; j < nplanes + R; ++j) {  // centres xs..xe-1 and fronts up to xe-1+R
-            const int s = j % NS;
-            if (j >= NS && (*(volatile int *)&sh.abort ||
-                            !mbar_wait(smem_u32(&bars[NS + s]), (unsigned)((j / NS - 1) & 1)))) {
+            if (refills > 0 && (*(volatile int *)&sh.abort || !mbar_wait(smem_u32(&bars[NS + s]), (refills - 1) & 1))) {
                 sh.abort = 1;
                 break;
             }
             const unsigned full = smem_u32(&bars[s]);
             unsigned char *sp = smem + s * S::bytes;
             const bool pw = CF::PS > 0 && j >= R;
-            unsigned tx = S::tx + (pw ? CF::pbytes : 0u);
-            if (j == R && t.z0 == 0 && t.vb == 0 && t.xs == 0 && t.half == 0) tx += a.fault_tx;
-            mbar_expect_tx(full, tx);
+            mbar_expect_tx(full, S::tx + (pw ? CF::pbytes : 0u) + (j == R ? fault_tx : 0u));
             // past the last plane it wraps (periodic) or, in a slab, comes from
             // the halo buffer's right planes (box plane x - nx + R).  Boxes
             // start at plane xs >= 0, so the left halo is never a box.
             const int xl = t.xs + j;  // < nx + R < 2 nx
             const bool hal = xl >= nx && halo;
-            const int x = hal ? xl - nx + R : xl >= nx ? xl - nx : xl;
-            // 1 piece, or 2-3 where the periodic z wrap cuts the box
-            int zstart = t.z0 - R, dst = 0;
-            while (dst < ZR) {
-                const int zw = zstart < 0 ? zstart + nz : (zstart >= nz ? zstart - nz : zstart);
-                int len = nz - zw;
-                if (len > ZR - dst) len = ZR - dst;
-                const CUtensorMap *m = len == ZR        ? (hal ? &maps.hzr : &maps.zr)
-                                       : len == TZ + R ? (hal ? &maps.htzr : &maps.tzr)
-                                       : len == TZ     ? (hal ? &maps.htz : &maps.tz)
-                                                       : (hal ? &maps.hr : &maps.r);
-                tma_load_4d(smem_u32(sp + S::box + dst * 4 * S::VB * sizeof(T)), m, c0, c1, zw, x, full);
-                zstart += len;
-                dst += len;
-            }
+            const int x = hal ? xl - nx + R : xl >= nx ? xl - nx : xl, h = hal ? TmaMaps::kHalo : 0;
+            tma_load_4d(smem_u32(sp + S::box), piece1 + h, c0, c1, za, x, full);
+            if (cut < ZR)
+                tma_load_4d(smem_u32(sp + S::box + cut * 4 * S::VB * (int)sizeof(T)), piece2 + h, c0, c1, 0, x, full);
             // the cell moments are read at a box's centre use, which is always an
             // interior plane; a halo box (front use only) loads plane nx-1's, unread
-            const int xm = hal ? nx - 1 : x;
-            bulk_load(smem_u32(sp + S::mb), a.mom_in + ((long long)xm * nz + t.z0) * NMOM, 8u * TZ * NMOM, full);
-            if (pw)
-                tma_load_4d(smem_u32(smem + CF::ring + (j - R) % CF::PSM * CF::pbytes), CF::PU ? &maps.pu : &maps.pa, c0,
-                            c1, t.z0, t.xs + j - R, full);
+            bulk_load(smem_u32(sp + S::mb), mom + (long long)(hal ? nx - 1 : x) * nz * NMOM, 8u * TZ * NMOM, full);
+            if (pw) {
+                tma_load_4d(smem_u32(smem + CF::ring + ps * CF::pbytes), CF::PU ? &maps.pu : &maps.pa, c0, c1, t.z0,
+                            t.xs + j - R, full);
+                ps = ps + 1 < CF::PSM ? ps + 1 : 0;
+            }
+            if (++s == NS) s = 0, ++refills;
             issued = j + 1;
         }
     }
@@ -474,6 +531,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     // RAG: where both rows are the tile before's the warp only takes its part in the
     // ring; where the first is (keep0 false) the second alone is stored
     const bool keep0 = !RAG || t.skip <= r;
+    const int put[RW] = {vact && keep0, vact}, sink = !keep0 && lane == 0;
     __syncthreads();  // the barriers are initialised
     if (RAG && t.skip >= r + RW) {
         for (int j = 0; j < nboxes; ++j) {
@@ -497,15 +555,14 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         for (int b = 0; b < R; ++b) {
             const int pl = xs - R + b;
             const bool hal = halo != nullptr && pl < 0;
-            const long long o = (long long)wrap_index(pl, g.nx) * P + own;
+            const int px = pl >= 0 ? pl : hal ? pl + R : pl + g.nx;  // (xs >= 0, nx > R)
+            const T *src = (hal ? halo + (long long)half * 8 * R * P : in) + ((long long)px * P + own);
+            long long step = hal ? 2 * R * P : fs;
+            asm volatile("" : "+l"(src), "+l"(step));  // one code for both sources
 #pragma unroll
             for (int f = 0; f < 4; ++f)
 #pragma unroll
-                for (int w = 0; w < RW; ++w) {
-                    const T *src = (hal ? halo + halo_offset(4 * half + f, pl, g.nx, R, P) + own : in + f * fs + o) +
-                                   w * g.nvs;
-                    pre[b][f][w] = vact ? O::ld(src) : O::zero();
-                }
+                for (int w = 0; w < RW; ++w) pre[b][f][w] = O::ldg(src + f * step + w * g.nvs, vact);
         }
     }
 
@@ -558,7 +615,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     const V kc = O::splat((R == 3 ? -20.0 : 6.0) * (a.c.kz + a.c.kx));  // centre weight of both axes
     const V cA = O::splat(a.cA), cY = O::splat(a.cY);
     const V p2s = O::splat(2 * a.c.pmo * a.c.st), p2c = O::splat(2 * a.c.pmo * a.c.ct), ps = O::splat(a.c.pmo * a.c.st);
-    const bool vac = VAC && a.c.pmo != 0.0;  // batched launches: instances without a vacuum term skip it
+    const bool vac = VAC && (!SA || a.c.pmo != 0.0);  // a batch's instances without a vacuum term skip it
 
     // x stencil in transposed form: xs[f][row][k] is the partial sum of the
     // centre plane (front - R + k) over the planes before the front.  A front
@@ -604,7 +661,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         for (int f = 0; f < 4; ++f) {
             V zs[2 * R + RW];
 #pragma unroll
-            for (int k = 0; k < 2 * R + RW; ++k) zs[k] = O::ld(&box[((r + k) * 4 + f) * VB + NP * lane]);
+            for (int k = 0; k < 2 * R + RW; ++k) zs[k] = O::lds(&box[((r + k) * 4 + f) * VB + NP * lane]);
 #pragma unroll
             for (int w = 0; w < RW; ++w) {
                 const V F = zs[R + w];
@@ -624,15 +681,43 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         }
     };
 
-    for (int j = 0; j < nboxes; ++j) {
-        const int i = j - R, x = xs + i;  // centre plane completed by front j (none while j < R)
-        const unsigned ox = (unsigned)x * P32 + own32;  // element offset of (x, zr, v) within a field
-        const int sf = j % NS, sc = (j + NS - R) % NS;
-        if (!mbar_wait(smem_u32(&bars[sf]), (unsigned)((j / NS) & 1)) ||
-            ((j & 3) == 0 && *(volatile int *)&sh.abort)) {  // another warp's abort, looked at every 4th plane
-            sh.abort = 1;
-            break;
+    // box j has landed (false: a wait ran out, or another warp's did; looked at every 4th plane)
+    auto ready = [&](int j) {
+        if (mbar_wait(smem_u32(&bars[j % NS]), (unsigned)((j / NS) & 1)) && !((j & 3) == 0 && *(volatile int *)&sh.abort))
+            return true;
+        sh.abort = 1;
+        return false;
+    };
+    // the first R fronts complete no centre: a loop of their own, as a condition on j
+    // in one loop left it to the compiler whether to make two of it
+    bool ok = true;
+#pragma unroll 1
+    for (int j = 0; j < R; ++j) {
+        ok = ok && ready(j);
+        if (!ok) break;
+        const T *fb = (const T *)(smem + j % NS * S::bytes + S::box);
+        if constexpr (RHS) {
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int w = 0; w < RW; ++w) {
+                    auto &q = sx[f][w];
+#pragma unroll
+                    for (int k = 0; k + 1 < 2 * R; ++k) q[k] = q[k + 1];
+                    q[2 * R - 1] = O::lds(&fb[((r + R + w) * 4 + f) * VB + NP * lane]);
+                }
+        } else {
+            V y[4][RW];
+            front(fb, y);
         }
+    }
+#pragma unroll 1
+    for (int j = R; ok && j < nboxes; ++j) {
+        const int i = j - R, x = xs + i;  // centre plane completed by front j
+        const unsigned ox = (unsigned)x * P32 + own32;  // element offset of (x, zr, v) within a field
+        const int sf = j % NS, sc = i % NS;
+        ok = ready(j);
+        if (!ok) break;
         V y[4][RW], cen[4][RW];
         const T *fb = (const T *)(smem + sf * S::bytes + S::box);
         const unsigned char *sp = smem + sc * S::bytes;
@@ -642,20 +727,17 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
             for (int f = 0; f < 4; ++f) {
                 V zs[2 * R + RW];
 #pragma unroll
-                for (int k = 0; k < 2 * R + RW; ++k)
-                    if (j >= R) zs[k] = O::ld(&zb[((r + k) * 4 + f) * VB + NP * lane]);
+                for (int k = 0; k < 2 * R + RW; ++k) zs[k] = O::lds(&zb[((r + k) * 4 + f) * VB + NP * lane]);
 #pragma unroll
                 for (int w = 0; w < RW; ++w) {
-                    const V F = O::ld(&fb[((r + R + w) * 4 + f) * VB + NP * lane]);
+                    const V F = O::lds(&fb[((r + R + w) * 4 + f) * VB + NP * lane]);
                     auto &q = sx[f][w];
-                    if (j >= R) {
-                        V z7[2 * R + 1], x7[2 * R + 1];
+                    V z7[2 * R + 1], x7[2 * R + 1];
 #pragma unroll
-                        for (int k = 0; k <= 2 * R; ++k) z7[k] = zs[w + k], x7[k] = k < 2 * R ? q[k < 2 * R ? k : 0] : F;
-                        cen[f][w] = zs[R + w];
-                        y[f][w] = vadd(vfma(fz, adv_diff<T, R>(z7), vmul(fx, adv_diff<T, R>(x7))),
-                                       vfma(kz, ko_sum<T, R>(z7), vmul(kx, ko_sum<T, R>(x7))));
-                    }
+                    for (int k = 0; k <= 2 * R; ++k) z7[k] = zs[w + k], x7[k] = k < 2 * R ? q[k < 2 * R ? k : 0] : F;
+                    cen[f][w] = zs[R + w];
+                    y[f][w] = vadd(vfma(fz, adv_diff<T, R>(z7), vmul(fx, adv_diff<T, R>(x7))),
+                                   vfma(kz, ko_sum<T, R>(z7), vmul(kx, ko_sum<T, R>(x7))));
 #pragma unroll
                     for (int k = 0; k + 1 < 2 * R; ++k) q[k] = q[k + 1];
                     q[2 * R - 1] = F;
@@ -664,12 +746,11 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         } else {
             front(fb, y);
         }
-        if (j < R) continue;
         if constexpr (!RHS) {
 #pragma unroll
             for (int f = 0; f < 4; ++f)
 #pragma unroll
-                for (int w = 0; w < RW; ++w) cen[f][w] = O::ld(&zb[((r + R + w) * 4 + f) * VB + NP * lane]);
+                for (int w = 0; w < RW; ++w) cen[f][w] = O::lds(&zb[((r + R + w) * 4 + f) * VB + NP * lane]);
         }
         V pin[4][RW];  // the pointwise input: U (S2, S3) or B (S4)
         if (CF::PU || CF::PA) {
@@ -677,7 +758,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
 #pragma unroll
             for (int f = 0; f < 4; ++f)
 #pragma unroll
-                for (int w = 0; w < RW; ++w) pin[f][w] = O::ld(&pb[((r + w) * 4 + f) * VB + NP * lane]);
+                for (int w = 0; w < RW; ++w) pin[f][w] = O::lds(&pb[((r + w) * 4 + f) * VB + NP * lane]);
         }
         V outm[4][RW], outb[4][RW];
 #pragma unroll
@@ -731,30 +812,21 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                 }
             }
         }
-        if (vact && keep0) {
-            T *dp = (MODE == MODE_S4B || MODE == MODE_RHS ? rd<SA>(a.acc_dst) : rd<SA>(a.y_dst)) + hoff + ox;
+        T *dp = (MODE == MODE_S4B || MODE == MODE_RHS ? rd<SA>(a.acc_dst) : rd<SA>(a.y_dst)) + hoff + ox;
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+#pragma unroll
+            for (int w = 0; w < RW; ++w) O::st_if(dp + f * fs32 + w * g.nvs, outm[f][w], put[w]);
+        if (MODE == MODE_S2B) {
+            T *bp = rd<SA>(a.acc_dst) + hoff + ox;
 #pragma unroll
             for (int f = 0; f < 4; ++f)
 #pragma unroll
-                for (int w = 0; w < RW; ++w) O::st(dp + f * fs32 + w * g.nvs, outm[f][w]);
-            if (MODE == MODE_S2B) {
-                T *bp = rd<SA>(a.acc_dst) + hoff + ox;
-#pragma unroll
-                for (int f = 0; f < 4; ++f)
-#pragma unroll
-                    for (int w = 0; w < RW; ++w) O::st(bp + f * fs32 + w * g.nvs, outb[f][w]);
-            }
+                for (int w = 0; w < RW; ++w) O::st_if(bp + f * fs32 + w * g.nvs, outb[f][w], put[w]);
         }
-        if (RAG && !keep0) {
-            const long long o = hoff + ox + g.nvs;
-            T *dp = (MODE == MODE_S4B || MODE == MODE_RHS ? a.acc_dst : a.y_dst) + o;
+        if (RAG)
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                if (vact) O::st(dp + f * fs, outm[f][1]);
-                if (MODE == MODE_S2B && vact) O::st(a.acc_dst + o + f * fs, outb[f][1]);
-                if (lane == 0) *(volatile unsigned long long *)&sh.sink = O::bits(outm[f][0]);
-            }
-        }
+            for (int f = 0; f < 4; ++f) sink_if(smem_u32(&sh.sink), O::bits(outm[f][0]), sink);
         // The centre use is the box's last (a right-halo box has none: its slot is
         // not filled again).  The arrive comes after the stores: they need every
         // value this plane read from shared memory, so no such read can still be
@@ -823,14 +895,13 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     __syncthreads();
     const bool aborted = sh.abort != 0;
     if constexpr (MODE == MODE_RHS) {  // a caller without a status word sees an incomplete tile as NaN
-        if (aborted && vact)
+        if (aborted)
             for (int x = xs; x < t.xe; ++x)
 #pragma unroll
                 for (int f = 0; f < 4; ++f)
 #pragma unroll
                     for (int w = 0; w < RW; ++w)
-                        if (w > 0 || keep0)
-                            O::st(a.acc_dst + hoff + f * fs + (long long)x * P + own + w * g.nvs, O::splat(nan("")));
+                        O::st_if(a.acc_dst + hoff + f * fs + (long long)x * P + own + w * g.nvs, O::splat(nan("")), put[w]);
     }
     return aborted;
 }
@@ -949,7 +1020,6 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
                     // through the generic proxy (a host copy when the work-list was built)
                     tensormap_acquire(&e.maps.zr);
                     tensormap_acquire(&e.maps.tzr);
-                    tensormap_acquire(&e.maps.tz);
                     tensormap_acquire(&e.maps.r);
                     if (MarchCfg<T, R, MODE, TZ>::PU) tensormap_acquire(&e.maps.pu);
                     if (MarchCfg<T, R, MODE, TZ>::PA) tensormap_acquire(&e.maps.pa);
@@ -983,6 +1053,7 @@ __global__ void __launch_bounds__(threads_of(TZ), tma_ctas_per_sm<T, TZ>())
 // one).  The wait gives up after `spins` polls; the kernel then records the
 // timeout in the status word, as a march does, invalidates the barrier and
 // returns.  Nothing else is touched, so the context stays usable.
+#if NUOSC_PART == 0
 __global__ void k_wait_selftest(int *status, unsigned spins) {
     __shared__ __align__(8) unsigned long long bar;
     if (threadIdx.x == 0) {
@@ -998,6 +1069,7 @@ cudaError_t launch_wait_selftest(int *status, unsigned spins, cudaStream_t s) {
     k_wait_selftest<<<1, 32, 0, s>>>(status, spins);
     return cudaGetLastError();
 }
+#endif
 
 // ------------------------------------------------------------------ host side
 namespace {
@@ -1064,16 +1136,16 @@ template <typename T>
 bool make_maps(TmaMaps *m, const StageArgs<T> &a, int tz, int r) {
     memset((void *)&m->pu, 0, sizeof m->pu);
     memset((void *)&m->pa, 0, sizeof m->pa);
-    memset((void *)&m->hzr, 0, 4 * sizeof m->hzr);
+    memset((void *)&m->hzr, 0, 3 * sizeof m->hzr);
     // a slab's halo buffer as a register of 2R planes
     Geom h = a.g;
     h.nx = 2 * r;
     h.fs = (long long)h.nx * h.nz * h.nvs;
     return make_map<T>(&m->zr, a.in, a.g, tz + 2 * r) && make_map<T>(&m->tzr, a.in, a.g, tz + r) &&
-           make_map<T>(&m->tz, a.in, a.g, tz) && make_map<T>(&m->r, a.in, a.g, r) &&
+           make_map<T>(&m->r, a.in, a.g, r) &&
            (!a.u || make_map<T>(&m->pu, a.u, a.g, tz)) && (!a.acc_src || make_map<T>(&m->pa, a.acc_src, a.g, tz)) &&
            (!a.halo || (make_map<T>(&m->hzr, a.halo, h, tz + 2 * r) && make_map<T>(&m->htzr, a.halo, h, tz + r) &&
-                        make_map<T>(&m->htz, a.halo, h, tz) && make_map<T>(&m->hr, a.halo, h, r)));
+                        make_map<T>(&m->hr, a.halo, h, r)));
 }
 
 template <typename T, int R, int MODE, int TZ, bool VAC, bool M64>
@@ -1103,12 +1175,17 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     return e;
 }
 
+}  // namespace
+
+// The launchers below are instantiated in parts 1 to 10.
 template <typename T, int TZ>
 cudaError_t launch_rhs_t(const StageArgs<T> &a, bool ko6, XTile t, cudaStream_t s) {
     if (a.c.pmo != 0.0)
         return ko6 ? launch_t<T, 3, MODE_RHS, TZ, true, true>(a, t, s) : launch_t<T, 2, MODE_RHS, TZ, true, true>(a, t, s);
     return ko6 ? launch_t<T, 3, MODE_RHS, TZ, false, true>(a, t, s) : launch_t<T, 2, MODE_RHS, TZ, false, true>(a, t, s);
 }
+
+namespace {
 
 template <typename T, int R, int TZ, bool VAC, bool M64>
 cudaError_t launch_tm(const StageArgs<T> &a, int mode, XTile t, cudaStream_t s) {
@@ -1121,19 +1198,15 @@ cudaError_t launch_tm(const StageArgs<T> &a, int mode, XTile t, cudaStream_t s) 
     }
 }
 
+}  // namespace
+
 template <typename T, int R, int TZ, bool M64>
 cudaError_t launch_tv(const StageArgs<T> &a, int mode, XTile t, cudaStream_t s) {
     return a.c.pmo != 0.0 ? launch_tm<T, R, TZ, true, M64>(a, mode, t, s)
                           : launch_tm<T, R, TZ, false, M64>(a, mode, t, s);
 }
 
-// moment partials summed in FP64 (always for FP64 state; for FP32 state per
-// the tile's msum) or in float within a velocity block
-template <typename T, int R, int TZ>
-cudaError_t launch_tms(const StageArgs<T> &a, int mode, XTile t, cudaStream_t s) {
-    if constexpr (sizeof(T) == 8) return launch_tv<T, R, TZ, true>(a, mode, t, s);
-    else return t.msum ? launch_tv<T, R, TZ, true>(a, mode, t, s) : launch_tv<T, R, TZ, false>(a, mode, t, s);
-}
+namespace {
 
 // ---- batched launch: one persistent grid per stage over many instances
 template <typename T, int R, int MODE, int TZ>
@@ -1189,6 +1262,75 @@ struct BatchLaunch {
         return batch_launch_t<T, R, MODE, TZ, VAC, M64>(items, starts, n, ntiles, counter, halt, grid, s);
     }
 };
+
+}  // namespace
+
+template <typename T, bool M64>
+int batch_grid_m(int mode, bool ko6, int tz, bool vac, int device) {
+    return batch_dispatch<T, M64, BatchGrid>(mode, ko6, tz, vac, device);
+}
+
+template <typename T, bool M64>
+cudaError_t batch_launch_m(const void *items, const long long *starts, int n, long long ntiles,
+                           unsigned long long *counter, const int *halt, int mode, bool ko6, int tz, bool vac, int grid,
+                           cudaStream_t s) {
+    return batch_dispatch<T, M64, BatchLaunch>(mode, ko6, tz, vac, items, starts, n, ntiles, counter, halt, grid, s);
+}
+
+#define NUOSC_STAGES(X, T, R, M64)                                                          \
+    X template cudaError_t launch_tv<T, R, 16, M64>(const StageArgs<T> &, int, XTile, cudaStream_t); \
+    X template cudaError_t launch_tv<T, R, 8, M64>(const StageArgs<T> &, int, XTile, cudaStream_t);
+#define NUOSC_RHS(X, T)                                                                   \
+    X template cudaError_t launch_rhs_t<T, 16>(const StageArgs<T> &, bool, XTile, cudaStream_t);    \
+    X template cudaError_t launch_rhs_t<T, 8>(const StageArgs<T> &, bool, XTile, cudaStream_t);
+#define NUOSC_BATCH(X, T, M64)                                                              \
+    X template int batch_grid_m<T, M64>(int, bool, int, bool, int);                                   \
+    X template cudaError_t batch_launch_m<T, M64>(const void *, const long long *, int, long long,    \
+                                                  unsigned long long *, const int *, int, bool, int, \
+                                                  bool, int, cudaStream_t);
+#if NUOSC_PART == 1
+NUOSC_STAGES(, double, 3, true)
+#elif NUOSC_PART == 2
+NUOSC_STAGES(, double, 2, true)
+#elif NUOSC_PART == 3
+NUOSC_STAGES(, float, 3, true)
+#elif NUOSC_PART == 4
+NUOSC_STAGES(, float, 2, true)
+#elif NUOSC_PART == 5
+NUOSC_STAGES(, float, 3, false)
+#elif NUOSC_PART == 6
+NUOSC_STAGES(, float, 2, false)
+#elif NUOSC_PART == 7
+NUOSC_RHS(, double)
+NUOSC_RHS(, float)
+#elif NUOSC_PART == 8
+NUOSC_BATCH(, double, true)
+#elif NUOSC_PART == 9
+NUOSC_BATCH(, float, true)
+#elif NUOSC_PART == 10
+NUOSC_BATCH(, float, false)
+#else  // part 0: the host side, to the end of the file
+NUOSC_STAGES(extern, double, 3, true)
+NUOSC_STAGES(extern, double, 2, true)
+NUOSC_STAGES(extern, float, 3, true)
+NUOSC_STAGES(extern, float, 2, true)
+NUOSC_STAGES(extern, float, 3, false)
+NUOSC_STAGES(extern, float, 2, false)
+NUOSC_RHS(extern, double)
+NUOSC_RHS(extern, float)
+NUOSC_BATCH(extern, double, true)
+NUOSC_BATCH(extern, float, true)
+NUOSC_BATCH(extern, float, false)
+
+namespace {
+
+// moment partials summed in FP64 (always for FP64 state; for FP32 state per
+// the tile's msum) or in float within a velocity block
+template <typename T, int R, int TZ>
+cudaError_t launch_tms(const StageArgs<T> &a, int mode, XTile t, cudaStream_t s) {
+    if constexpr (sizeof(T) == 8) return launch_tv<T, R, TZ, true>(a, mode, t, s);
+    else return t.msum ? launch_tv<T, R, TZ, true>(a, mode, t, s) : launch_tv<T, R, TZ, false>(a, mode, t, s);
+}
 
 }  // namespace
 
@@ -1271,10 +1413,10 @@ long long xtma_batch_fill(void *item, const StageArgs<T> &a, bool ko6, int tz, i
 template <typename T>
 int xtma_batch_grid(int mode, bool ko6, int tz, bool vac, bool m64, int device) {
     if ((tz != 8 && tz != 16) || !tma_mode(mode)) return -1;
-    if constexpr (sizeof(T) == 8) return batch_dispatch<T, true, BatchGrid>(mode, ko6, tz, vac, device);
+    if constexpr (sizeof(T) == 8) return batch_grid_m<T, true>(mode, ko6, tz, vac, device);
     else
-        return m64 ? batch_dispatch<T, true, BatchGrid>(mode, ko6, tz, vac, device)
-                   : batch_dispatch<T, false, BatchGrid>(mode, ko6, tz, vac, device);
+        return m64 ? batch_grid_m<T, true>(mode, ko6, tz, vac, device)
+                   : batch_grid_m<T, false>(mode, ko6, tz, vac, device);
 }
 
 template <typename T>
@@ -1284,13 +1426,10 @@ cudaError_t launch_stage_xtma_batch(const void *items, const long long *starts, 
     if ((tz != 8 && tz != 16) || !tma_mode(mode) || n < 1 || grid < 1)
         return cudaErrorInvalidValue;
     if constexpr (sizeof(T) == 8)
-        return batch_dispatch<T, true, BatchLaunch>(mode, ko6, tz, vac, items, starts, n, ntiles, counter, halt, grid,
-                                                    s);
+        return batch_launch_m<T, true>(items, starts, n, ntiles, counter, halt, mode, ko6, tz, vac, grid, s);
     else
-        return m64 ? batch_dispatch<T, true, BatchLaunch>(mode, ko6, tz, vac, items, starts, n, ntiles, counter, halt,
-                                                          grid, s)
-                   : batch_dispatch<T, false, BatchLaunch>(mode, ko6, tz, vac, items, starts, n, ntiles, counter,
-                                                           halt, grid, s);
+        return m64 ? batch_launch_m<T, true>(items, starts, n, ntiles, counter, halt, mode, ko6, tz, vac, grid, s)
+                   : batch_launch_m<T, false>(items, starts, n, ntiles, counter, halt, mode, ko6, tz, vac, grid, s);
 }
 
 template <typename T>
@@ -1372,5 +1511,7 @@ template cudaError_t launch_stage_xtma_batch<double>(const void *, const long lo
 template cudaError_t launch_stage_xtma_batch<float>(const void *, const long long *, int, long long,
                                                     unsigned long long *, const int *, int, bool, int, bool, bool,
                                                     int, cudaStream_t);
+
+#endif  // NUOSC_PART
 
 }  // namespace nuosc
