@@ -270,21 +270,23 @@ cudaError_t launch_init(T *reg, const double *G0, const double *G0b, Geom g, int
 // (with 1 and 8 the advection test's integrals I1, I2, nuosc_ana.cpp:58-61).
 // ----------------------------------------------------------------------------
 //
-// A warp keeps one chunk of velocities (32 lanes x 16 bytes) and strides over the
-// cells, so the spectra, their reciprocals and the weights stay in registers and a
-// point costs its two square roots and the sums, no divide.  Time of the whole
-// analysis() call, one value per load with two divides per point -> this:
-//   64x64x162 FP64 74 -> 37 us, 128x128x642 228 -> 157, 512x256x642 1247 -> 995 (830
-//   of them the state at the copy bandwidth), 256x256x642 FP32 630 -> 569.
+// A thread keeps one 16-byte vector of velocities (rows are whole vectors, so the
+// threads of a warp read consecutive addresses, across row ends too, and none
+// idles where a row is short) and strides over the cells: the spectra, their
+// reciprocals and the weights stay in registers and a point costs its two square
+// roots and the sums, no divide.  Time of the whole analysis() call, with one value
+// per load and two divides per point -> with a warp per chunk of 32 vectors -> this:
+//   512x256, FP64, 12 velocities 119 -> 94 -> 44 us, 642: 1233 -> 983 -> 922 (830 of
+//   them the state at the copy bandwidth); FP32, 12: 98 -> 168 -> 44 (3 of a chunk's
+//   32 lanes had work), 162: 370 -> 388 -> 266; 16x16, FP64, 162: 69 -> 32 -> 31.
 template <typename T>
 __global__ void __launch_bounds__(256) k_analysis(const T *__restrict__ st, const double *__restrict__ G0,
                                                   const double *__restrict__ G0b, const double *__restrict__ vw,
                                                   Geom g, double *__restrict__ part) {
     constexpr int N = 16 / (int)sizeof(T);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nchunk = (g.nvs + 32 * N - 1) / (32 * N), nwarp = gridDim.x * 8, w = blockIdx.x * 8 + warp;
-    const int chunk = w % nchunk, first = w / nchunk, stride = (nwarp - chunk + nchunk - 1) / nchunk;
-    const int v = chunk * 32 * N + lane * N;
+    const int nvec = g.nvs / N, t = blockIdx.x * 256 + threadIdx.x;  // (at most 20,481 vectors)
+    const int stride = gridDim.x * 256 / nvec, first = t / nvec, v = (t - first * nvec) * N;
     double G[N], Gb[N], iG[N], iGb[N], wv[N];
 #pragma unroll
     for (int p = 0; p < N; ++p) {
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(256) k_analysis(const T *__restrict__ st, cons
 #pragma unroll
     for (int k = 0; k < ANA_NQ; ++k) q[k] = 0.0;
     long long cells = 0;
-    if (v < g.nv)
+    if (first < stride)
         for (long long cell = first; cell < g.ncell; cell += stride, ++cells) {
             const T *row = st + cell * g.nvs + v;
             double f[NF][N];
