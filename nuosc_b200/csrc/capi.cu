@@ -304,11 +304,12 @@ int run_stage_direct(nuosc_handle *h, int mode, int in, int u, int acc_src, int 
     const int ps = h->prof_begin(prof_kind(mode));
     if (mode == MODE_RHS && (h->kernel == NUOSC_KERNEL_AUTO || h->kernel == NUOSC_KERNEL_XTMA) &&
         rhs_xtma_fits<T>(h->g, a.in, a.acc_dst))
-        CUDA_TRY(launch_rhs_xtma<T>(a, h->ko6, h->stream));  // (and its tail, when there is one)
-    else
+        CUDA_TRY(launch_rhs_xtma<T>(a, h->ko6, &h->launches, h->stream));
+    else {
         CUDA_TRY(launch_stage_direct<T>(a, mode, h->ko6, h->stream));
+        h->launches++;
+    }
     h->prof_end(ps);
-    h->launches++;
     return 0;
 }
 
@@ -344,17 +345,19 @@ int run_stage_xmarch(nuosc_handle *h, bool tma, const XTile &tile, int mode, int
     const bool early = march && !h->halo && xtma_waves<T>(h->g, tile, h->sms) == 1;
     if (tma && !march) {
         CUDA_TRY(launch_stage_tail<T>(a, mode, h->ko6, 0, 1, h->stream));
+        h->launches++;
     } else if (tma) {
-        CUDA_TRY(launch_stage_xtma<T>(a, mode, h->ko6, tile, early, h->stream));
+        CUDA_TRY(launch_stage_xtma<T>(a, mode, h->ko6, tile, early, &h->launches, h->stream));
     } else {
         CUDA_TRY(launch_stage_xmarch<T>(a, mode, h->ko6, tile, h->stream));
+        h->launches++;
     }
     h->prof_end(ps);
     ps = h->prof_begin(5);
     const int nvb = tma ? xtma_num_vblocks<T>(h->g) : xmarch_num_vblocks(h->g, tile);
     CUDA_TRY(launch_moment_finalize(h->d_part, h->d_mom, h->g, nvb, early, h->stream));
     h->prof_end(ps);
-    h->launches += 2;
+    h->launches++;
     h->mom_valid = true;  // d_mom now holds the moments of the register this stage wrote
     return 0;
 }

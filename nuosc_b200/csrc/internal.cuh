@@ -164,6 +164,7 @@ struct XTile {
     int kind = 0;  // preferred x-march kernel from the tile table: 2 cp.async, 3 TMA, 0 either
     int msum = 1;  // FP32 TMA march: moment partials summed in FP64 (1) or in float within a block (0)
     bool early = false;  // of one launch: it is a single wave (xtma_waves)
+    long long *launched = nullptr;  // of one launch: where its kernels are counted
 };
 template <typename T>
 bool xmarch_supported(const Geom &g, bool ko6, XTile t);
@@ -179,9 +180,12 @@ bool xtma_supported(const Geom &g, XTile t);
 // x planes per CTA for grid g on a device of `sms` SMs
 template <typename T>
 int xtma_lx(const Geom &g, int tz, int sms);
-// The stage, the tail velocities included; not for grids with xtma_all_tail
+// The stage, the tail velocities included; not for grids with xtma_all_tail.  The
+// launchers of the march add the kernels they start (one, or two with a tail
+// kernel) to *launched.
 template <typename T>
-cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, bool early, cudaStream_t s);
+cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, bool early, long long *launched,
+                              cudaStream_t s);
 // waves of CTAs (a tail column included) of the stage's launch on `sms` SMs.  One:
 // all CTAs are resident at once, and the kernel after it may be launched, and wait,
 // while it runs (with more, waiting CTAs would take SMs from the ones still to come)
@@ -195,7 +199,7 @@ bool xtma_all_tail(const Geom &g);
 template <typename T>
 bool rhs_xtma_fits(const Geom &g, const void *in, const void *out);
 template <typename T>
-cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, cudaStream_t s);
+cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, long long *launched, cudaStream_t s);
 // velocity blocks of the TMA kernel's moment partials (32 velocities per block in FP64, 64 in FP32)
 template <typename T>
 int xtma_num_vblocks(const Geom &g);

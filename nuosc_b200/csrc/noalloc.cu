@@ -143,7 +143,7 @@ extern "C" int nuosc_calrhs_noalloc(const nuosc_rhs_desc *d, const void *in, voi
         a.cA = 1.0;
         e = launch_moments<double>(a.in, scratch, q, g, s);
         if (e == cudaSuccess)
-            e = rhs_xtma_fits<double>(g, in, out) ? launch_rhs_xtma<double>(a, ko6, s)
+            e = rhs_xtma_fits<double>(g, in, out) ? launch_rhs_xtma<double>(a, ko6, nullptr, s)
                                                   : launch_stage_direct<double>(a, MODE_RHS, ko6, s);
     } else {
         StageArgs<float> a{};
@@ -156,7 +156,7 @@ extern "C" int nuosc_calrhs_noalloc(const nuosc_rhs_desc *d, const void *in, voi
         a.cA = 1.0;
         e = launch_moments<float>(a.in, scratch, q, g, s);
         if (e == cudaSuccess)
-            e = rhs_xtma_fits<float>(g, in, out) ? launch_rhs_xtma<float>(a, ko6, s)
+            e = rhs_xtma_fits<float>(g, in, out) ? launch_rhs_xtma<float>(a, ko6, nullptr, s)
                                                  : launch_stage_direct<float>(a, MODE_RHS, ko6, s);
     }
     if (e != cudaSuccess) return fail(NUOSC_ERR_CUDA, cudaGetErrorString(e));

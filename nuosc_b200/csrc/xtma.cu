@@ -1170,6 +1170,7 @@ cudaError_t launch_t(const StageArgs<T> &a, XTile t, cudaStream_t s) {
     const StageTail f{nvbm, v0, tail_lanes(a.g.nvs - v0), t.early};
     e = launch_dependent(t.early, kern, grid, threads_of(TZ), smem, s, maps, a, zt, t.lx, nvb, f);
     if (e == cudaSuccess && tail && !column) e = launch_stage_tail<T>(a, MODE, R == 3, v0, nvb, s);
+    if (t.launched) *t.launched += tail && !column ? 2 : 1;
     return e;
 }
 
@@ -1447,8 +1448,10 @@ int xtma_tail_v0(const Geom &g) {
 }
 
 template <typename T>
-cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, bool early, cudaStream_t s) {
+cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t, bool early, long long *launched,
+                              cudaStream_t s) {
     t.early = early;
+    t.launched = launched;
     if (!a.mom_part || !xtma_fits<T>(a.g, t)) return cudaErrorInvalidValue;
     if (t.tz == 16) return ko6 ? launch_tms<T, 3, 16>(a, mode, t, s) : launch_tms<T, 2, 16>(a, mode, t, s);
     return ko6 ? launch_tms<T, 3, 8>(a, mode, t, s) : launch_tms<T, 2, 8>(a, mode, t, s);
@@ -1468,19 +1471,23 @@ bool rhs_xtma_fits(const Geom &g, const void *in, const void *out) {
 }
 
 template <typename T>
-cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, cudaStream_t s) {
+cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, long long *launched, cudaStream_t s) {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int tz = a.g.nz >= 22 ? 16 : 8;
-    const XTile t{tz, xtma_lx<T>(a.g, tz, sms), vblock<T>()};
-    if (xtma_all_tail<T>(a.g)) return launch_stage_tail<T>(a, MODE_RHS, ko6, 0, 1, s);
+    XTile t{tz, xtma_lx<T>(a.g, tz, sms), vblock<T>()};
+    t.launched = launched;
+    if (xtma_all_tail<T>(a.g)) {
+        if (launched) ++*launched;
+        return launch_stage_tail<T>(a, MODE_RHS, ko6, 0, 1, s);
+    }
     return tz == 16 ? launch_rhs_t<T, 16>(a, ko6, t, s) : launch_rhs_t<T, 8>(a, ko6, t, s);
 }
 
 template bool rhs_xtma_fits<double>(const Geom &, const void *, const void *);
 template bool rhs_xtma_fits<float>(const Geom &, const void *, const void *);
-template cudaError_t launch_rhs_xtma<double>(const StageArgs<double> &, bool, cudaStream_t);
-template cudaError_t launch_rhs_xtma<float>(const StageArgs<float> &, bool, cudaStream_t);
+template cudaError_t launch_rhs_xtma<double>(const StageArgs<double> &, bool, long long *, cudaStream_t);
+template cudaError_t launch_rhs_xtma<float>(const StageArgs<float> &, bool, long long *, cudaStream_t);
 template bool xtma_supported<double>(const Geom &, XTile);
 template bool xtma_fits<double>(const Geom &, XTile);
 template int xtma_lx<double>(const Geom &, int, int);
@@ -1495,8 +1502,10 @@ template int xtma_tail_v0<double>(const Geom &);
 template bool xtma_all_tail<double>(const Geom &);
 template bool xtma_all_tail<float>(const Geom &);
 template int xtma_tail_v0<float>(const Geom &);
-template cudaError_t launch_stage_xtma<double>(const StageArgs<double> &, int, bool, XTile, bool, cudaStream_t);
-template cudaError_t launch_stage_xtma<float>(const StageArgs<float> &, int, bool, XTile, bool, cudaStream_t);
+template cudaError_t launch_stage_xtma<double>(const StageArgs<double> &, int, bool, XTile, bool, long long *,
+                                               cudaStream_t);
+template cudaError_t launch_stage_xtma<float>(const StageArgs<float> &, int, bool, XTile, bool, long long *,
+                                              cudaStream_t);
 template size_t xtma_batch_item_bytes<double>();
 template size_t xtma_batch_item_bytes<float>();
 template long long xtma_batch_fill<double>(void *, const StageArgs<double> &, bool, int, int);
