@@ -302,7 +302,8 @@ int run_stage_direct(nuosc_handle *h, int mode, int in, int u, int acc_src, int 
         h->launches++;
     }
     const int ps = h->prof_begin(prof_kind(mode));
-    if (mode == MODE_RHS && (h->kernel == NUOSC_KERNEL_AUTO || h->kernel == NUOSC_KERNEL_XTMA) &&
+    if (mode == MODE_RHS &&
+        (h->kernel == NUOSC_KERNEL_XTMA || (h->kernel == NUOSC_KERNEL_AUTO && rhs_xtma_pays(h->g, h->ko6))) &&
         rhs_xtma_fits<T>(h->g, a.in, a.acc_dst))
         CUDA_TRY(launch_rhs_xtma<T>(a, h->ko6, &h->launches, h->stream));
     else {

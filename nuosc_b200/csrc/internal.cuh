@@ -198,6 +198,8 @@ bool xtma_all_tail(const Geom &g);
 // march, for grids and buffers it fits
 template <typename T>
 bool rhs_xtma_fits(const Geom &g, const void *in, const void *out);
+// whether it is the faster kernel there
+bool rhs_xtma_pays(const Geom &g, bool ko6);
 template <typename T>
 cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, long long *launched, cudaStream_t s);
 // velocity blocks of the TMA kernel's moment partials (32 velocities per block in FP64, 64 in FP32)

@@ -13,8 +13,8 @@
 // holds that array (6 MiB) until the process exits.
 //
 // The kernels are the library's own moment pass (kernels.cu) and the TMA march
-// (xtma.cu) -- or the direct stage kernel, for grids with nz < 14 and buffers
-// whose rows are not 16-byte aligned; only the scratch pointer differs.
+// (xtma.cu) -- or the direct stage kernel, for grids with nz < 14, buffers whose
+// rows are not 16-byte aligned and the smallest calls; only the scratch pointer differs.
 #include "../../include/nuosc_b200.h"
 #include "internal.cuh"
 
@@ -143,7 +143,8 @@ extern "C" int nuosc_calrhs_noalloc(const nuosc_rhs_desc *d, const void *in, voi
         a.cA = 1.0;
         e = launch_moments<double>(a.in, scratch, q, g, s);
         if (e == cudaSuccess)
-            e = rhs_xtma_fits<double>(g, in, out) ? launch_rhs_xtma<double>(a, ko6, nullptr, s)
+            e = rhs_xtma_pays(g, ko6) && rhs_xtma_fits<double>(g, in, out)
+                    ? launch_rhs_xtma<double>(a, ko6, nullptr, s)
                                                   : launch_stage_direct<double>(a, MODE_RHS, ko6, s);
     } else {
         StageArgs<float> a{};
@@ -156,7 +157,8 @@ extern "C" int nuosc_calrhs_noalloc(const nuosc_rhs_desc *d, const void *in, voi
         a.cA = 1.0;
         e = launch_moments<float>(a.in, scratch, q, g, s);
         if (e == cudaSuccess)
-            e = rhs_xtma_fits<float>(g, in, out) ? launch_rhs_xtma<float>(a, ko6, nullptr, s)
+            e = rhs_xtma_pays(g, ko6) && rhs_xtma_fits<float>(g, in, out)
+                    ? launch_rhs_xtma<float>(a, ko6, nullptr, s)
                                                  : launch_stage_direct<float>(a, MODE_RHS, ko6, s);
     }
     if (e != cudaSuccess) return fail(NUOSC_ERR_CUDA, cudaGetErrorString(e));

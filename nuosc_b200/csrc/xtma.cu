@@ -1461,7 +1461,7 @@ cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t
 // of the direct kernel's 13 or 9 loads per value from L2.  Whole call, moment
 // pass included: 128x128x642 FP64, KO6 1150 -> 567 us (140 of them the moment
 // pass); 250x130x162 FP32, KO4 296 -> 172 us.  The direct kernel stays for nz <
-// 14 and for buffers without 16-byte rows.
+// 14, for buffers without 16-byte rows and where rhs_xtma_pays says so.
 template <typename T>
 bool rhs_xtma_fits(const Geom &g, const void *in, const void *out) {
     // the tensor maps and the vector accesses need 16-byte aligned rows; a
@@ -1469,6 +1469,14 @@ bool rhs_xtma_fits(const Geom &g, const void *in, const void *out) {
     return g.nvs * sizeof(T) % 16 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 &&
            xtma_fits<T>(g, XTile{g.nz >= 22 ? 16 : 8, 0, vblock<T>()});
 }
+
+// The smallest calls are one latency chain (launch, constants, first box): the
+// direct kernel's is shorter with the 4th difference, its 9 loads per value in
+// flight at once.  Below 40,000 values a field, whole call, direct and march:
+// 16x16x42 FP32 9.1 and 10.5 us, 24x16x92 9.3 and 10.5, FP64 24x16x42 10.1 and 10.4;
+// 16x16x162 (41,472) FP32 12.3 and 11.1; 6th difference 16x16x42 10.3 and 10.5,
+// 24x16x92 FP64 12.3 and 10.5.
+bool rhs_xtma_pays(const Geom &g, bool ko6) { return ko6 || g.fs >= 40000; }
 
 template <typename T>
 cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, long long *launched, cudaStream_t s) {
