@@ -364,8 +364,8 @@ int run_stage_xmarch(nuosc_handle *h, bool tma, const XTile &tile, int mode, int
 }
 
 // stage-kernel path for this handle: 0 direct, 1 cp.async x-march, 2 TMA x-march (-1: unsupported request).
-// `tile` is the handle's tile, with 8-row tiles in place of 16-row ones when
-// nz only fits those (the TMA kernel is preferred at either height).
+// `tile` is the path's tile: the handle's, with 8-row tiles in place of 16-row ones
+// when nz only fits those (the TMA kernel is preferred at either height).
 template <typename T>
 int stage_path(nuosc_handle *h, XTile &tile) {
     tile = h->tile;
@@ -375,12 +375,16 @@ int stage_path(nuosc_handle *h, XTile &tile) {
         if (xtma_supported<T>(h->g, t8)) tile = t8;
     }
     const bool tma = xtma_supported<T>(h->g, tile), cpa = xmarch_supported<T>(h->g, h->ko6, h->tile);
+    auto cp_async = [&] {
+        tile = h->auto_lx ? xmarch_tile(h->g, h->tile, h->sms) : h->tile;
+        return 1;
+    };
     switch (h->kernel) {
     case NUOSC_KERNEL_DIRECT: return 0;
-    case NUOSC_KERNEL_XMARCH: return cpa ? 1 : -1;
+    case NUOSC_KERNEL_XMARCH: return cpa ? cp_async() : -1;
     case NUOSC_KERNEL_XTMA: return tma ? 2 : -1;
     default:
-        if (h->tile.kind == NUOSC_KERNEL_XMARCH && cpa) return 1;
+        if (h->tile.kind == NUOSC_KERNEL_XMARCH && cpa) return cp_async();
         if (tma) return 2;
         // nz is no multiple of 8: the TMA kernel with overlapping z tiles
         if (!h->halo) {
@@ -394,7 +398,7 @@ int stage_path(nuosc_handle *h, XTile &tile) {
                 }
             }
         }
-        return cpa ? 1 : 0;
+        return cpa ? cp_async() : 0;
     }
 }
 
@@ -495,7 +499,6 @@ int step_impl(nuosc_handle *h, int nsteps) {
     const int path = stage_path<T>(h, tile);
     if (path < 0) return fail(NUOSC_ERR_UNSUPPORTED, "the requested stage kernel does not support this geometry/tile");
     const bool xm = path > 0, tma = path == 2;
-    if (!tma) tile = h->tile;
     if (h->halo && !tma)
         return fail(NUOSC_ERR_UNSUPPORTED, "x-slabs of a decomposed solve run on the TMA kernel only (nz %% 8 == 0)");
     if (h->halo && h->px > 1)

@@ -168,6 +168,8 @@ struct XTile {
 };
 template <typename T>
 bool xmarch_supported(const Geom &g, bool ko6, XTile t);
+// its tile where the handle's is not the user's or the tile table's
+XTile xmarch_tile(const Geom &g, XTile t, int sms);
 template <typename T>
 cudaError_t launch_stage_xmarch(const StageArgs<T> &a, int mode, bool ko6, XTile t, cudaStream_t s);
 // TMA-fed variant of the x-march kernel (xtma.cu).  fits: it runs this grid

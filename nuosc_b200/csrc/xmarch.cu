@@ -351,6 +351,29 @@ bool xmarch_supported(const Geom &g, bool, XTile t) {
     return (t.tz == 4 || t.tz == 8 || t.tz == 16) && t.lx >= 1 && t.vb == VB && g.nx >= 4 && g.nz >= 1;
 }
 
+// 8 rows, two CTAs per SM: 16 were up to 2.2 times slower (us per FP64 step, 256x256
+// cells, 42 velocities, 24 planes: 993 against 1345; FP32 512x8x42 99 against 135).
+// Up to 48 planes a segment: it costs its planes and about 3 more, and a launch of
+// more than one wave of CTAs about half a wave beyond its work.  Measured, FP64, the
+// rule's lx in brackets: 512x8x42 [7] 8: 107, 16: 117, 32: 203; 100x90x42 [17] 8: 187,
+// 16: 181, 32: 212; 256x256x162 [32] 32: 3098, 48: 3078, 128: 3451, 256: 3872;
+// 20000x13x42 [48] 48: 4351, 64: 4341, 256: 5113.
+XTile xmarch_tile(const Geom &g, XTile t, int sms) {
+    const double per = (double)((g.nz + 7) / 8) * ((g.nvs + VB - 1) / VB) * 2;  // CTAs per segment
+    const int least = (g.nx + 32766) / 32767;                                   // (grid extent)
+    double cost = -1.0;
+    t.tz = 8;
+    for (int lx = least; lx <= 48 || lx == least; ++lx) {
+        const int nseg = (g.nx + lx - 1) / lx;
+        const double waves = per * nseg / (2.0 * sms), c = (waves <= 1.0 ? 1.0 : waves + 0.5) * (lx + 3);
+        if (cost < 0.0 || c < cost) {
+            cost = c;
+            t.lx = lx;
+        }
+    }
+    return t;
+}
+
 namespace {
 
 // deepest ring (4, 3 or 2 planes) that lets ctas_per_sm CTAs share the SM's 228 KB
