@@ -392,7 +392,7 @@ int stage_path(nuosc_handle *h, XTile &tile) {
                 XTile t = h->tile;
                 if (t.tz < tz) continue;
                 t.tz = tz;
-                if (xtma_fits<T>(h->g, t)) {
+                if (xtma_fits<T>(h->g, t) && xtma_grid_ok(h->g, t)) {
                     tile = t;
                     return 2;
                 }

@@ -179,6 +179,8 @@ template <typename T>
 bool xtma_fits(const Geom &g, XTile t);
 template <typename T>
 bool xtma_supported(const Geom &g, XTile t);
+// its launch has a grid the device takes (65,535 z tiles, 32,767 segments)
+bool xtma_grid_ok(const Geom &g, XTile t);
 // x planes per CTA for grid g on a device of `sms` SMs
 template <typename T>
 int xtma_lx(const Geom &g, int tz, int sms);

@@ -1348,6 +1348,10 @@ bool xtma_supported(const Geom &g, XTile t) {
     return g.nz % t.tz == 0 && xtma_fits<T>(g, t);
 }
 
+bool xtma_grid_ok(const Geom &g, XTile t) {
+    return (g.nz + t.tz - 1) / t.tz <= 65535 && (g.nx + t.lx - 1) / t.lx <= 32767;
+}
+
 // x planes per CTA.  A segment costs its planes plus about 10 more (the launch of
 // the CTA, the constants, R planes left of it and R right of it), and a launch
 // costs whole waves of CTAs, so the number of segments minimises waves x (lx +
@@ -1463,11 +1467,20 @@ cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t
 // pass); 250x130x162 FP32, KO4 296 -> 172 us.  The direct kernel stays for nz <
 // 14, for buffers without 16-byte rows and where rhs_xtma_pays says so.
 template <typename T>
+XTile rhs_tile(const Geom &g) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int tz = g.nz >= 22 ? 16 : 8;
+    return XTile{tz, xtma_lx<T>(g, tz, sms), vblock<T>()};
+}
+
+template <typename T>
 bool rhs_xtma_fits(const Geom &g, const void *in, const void *out) {
     // the tensor maps and the vector accesses need 16-byte aligned rows; a
     // caller's own buffers may have neither
     return g.nvs * sizeof(T) % 16 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0 &&
-           xtma_fits<T>(g, XTile{g.nz >= 22 ? 16 : 8, 0, vblock<T>()});
+           xtma_fits<T>(g, XTile{g.nz >= 22 ? 16 : 8, 0, vblock<T>()}) &&
+           ((g.nx <= 32767 && g.nz <= 65535) || xtma_grid_ok(g, rhs_tile<T>(g)));
 }
 
 // The smallest calls are one latency chain (launch, constants, first box): the
@@ -1480,16 +1493,13 @@ bool rhs_xtma_pays(const Geom &g, bool ko6) { return ko6 || g.fs >= 40000; }
 
 template <typename T>
 cudaError_t launch_rhs_xtma(const StageArgs<T> &a, bool ko6, long long *launched, cudaStream_t s) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int tz = a.g.nz >= 22 ? 16 : 8;
-    XTile t{tz, xtma_lx<T>(a.g, tz, sms), vblock<T>()};
+    XTile t = rhs_tile<T>(a.g);
     t.launched = launched;
     if (xtma_all_tail<T>(a.g)) {
         if (launched) ++*launched;
         return launch_stage_tail<T>(a, MODE_RHS, ko6, 0, 1, s);
     }
-    return tz == 16 ? launch_rhs_t<T, 16>(a, ko6, t, s) : launch_rhs_t<T, 8>(a, ko6, t, s);
+    return t.tz == 16 ? launch_rhs_t<T, 16>(a, ko6, t, s) : launch_rhs_t<T, 8>(a, ko6, t, s);
 }
 
 template bool rhs_xtma_fits<double>(const Geom &, const void *, const void *);
