@@ -617,7 +617,7 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
     const V p2s = O::splat(2 * a.c.pmo * a.c.st), p2c = O::splat(2 * a.c.pmo * a.c.ct), ps = O::splat(a.c.pmo * a.c.st);
     const bool vac = VAC && (!SA || a.c.pmo != 0.0);  // a batch's instances without a vacuum term skip it
 
-    // x stencil in transposed form: xs[f][row][k] is the partial sum of the
+    // x stencil in transposed form: sx[f][row][k] is the partial sum of the
     // centre plane (front - R + k) over the planes before the front.  A front
     // value F completes centre front - R and is added, with its tap's weight,
     // to the R..2R-1 others; the move to the next slot is the fma's own
@@ -653,30 +653,38 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
                 }
             }
         }
-    // front j of the march: box j's values enter the x sums and, with their z
-    // sums, the centre sum of their own plane; y = the completed stencil sums
-    // of centre j - R
+    // front j of the march: box j's values enter the x sums; y = the completed
+    // stencil sums of centre j - R.  In FP64 a value's own centre term and z sum enter
+    // with it, in one chain with the x sum.  In FP32 that chain's terms, up to 10 times
+    // the state, cost up to 1.4 times the error of a whole solve (a batch member 8.9e-8
+    // of the state after 60 steps, 6.3e-8 with the sums apart): there the z sum is
+    // formed by itself, when its plane is the centre, and the centre term comes last.
+    constexpr bool APART = sizeof(T) == 4;
     auto front = [&](const T *box, V (&y)[4][RW]) {
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
             V zs[2 * R + RW];
 #pragma unroll
-            for (int k = 0; k < 2 * R + RW; ++k) zs[k] = O::lds(&box[((r + k) * 4 + f) * VB + NP * lane]);
+            for (int k = APART ? R : 0; k < (APART ? R + RW : 2 * R + RW); ++k)
+                zs[k] = O::lds(&box[((r + k) * 4 + f) * VB + NP * lane]);
 #pragma unroll
             for (int w = 0; w < RW; ++w) {
                 const V F = zs[R + w];
                 auto &q = sx[f][w];
                 y[f][w] = vfma(tap(0), F, q[0]);
 #pragma unroll
-                for (int k = 0; k + 1 < 2 * R; ++k) q[k] = vfma(tap(k + 1), F, q[k + 1]);
+                for (int k = 0; k + 1 < 2 * R; ++k)
+                    q[k] = APART && k == R - 1 ? q[k + 1] : vfma(tap(k + 1), F, q[k + 1]);
                 q[2 * R - 1] = vmul(tap(2 * R), F);
-                V z = q[R - 1];
-                z = vfma(wz[0], zs[w + R - 2], z);
-                z = vfma(wz[1], zs[w + R - 1], z);
-                z = vfma(wz[2], zs[w + R + 1], z);
-                z = vfma(wz[3], zs[w + R + 2], z);
-                if (R == 3) z = vfma(kz, vadd(zs[w], zs[w + 2 * R]), z);
-                q[R - 1] = z;
+                if constexpr (!APART) {
+                    V z = q[R - 1];
+                    z = vfma(wz[0], zs[w + R - 2], z);
+                    z = vfma(wz[1], zs[w + R - 1], z);
+                    z = vfma(wz[2], zs[w + R + 1], z);
+                    z = vfma(wz[3], zs[w + R + 2], z);
+                    if (R == 3) z = vfma(kz, vadd(zs[w], zs[w + 2 * R]), z);
+                    q[R - 1] = z;
+                }
             }
         }
     };
@@ -748,9 +756,24 @@ __device__ __forceinline__ bool xtma_consume(const StageArgs<T> &a, const Tile &
         }
         if constexpr (!RHS) {
 #pragma unroll
-            for (int f = 0; f < 4; ++f)
+            for (int f = 0; f < 4; ++f) {
+                V zs[2 * R + RW];
 #pragma unroll
-                for (int w = 0; w < RW; ++w) cen[f][w] = O::lds(&zb[((r + R + w) * 4 + f) * VB + NP * lane]);
+                for (int k = APART ? 0 : R; k < (APART ? 2 * R + RW : R + RW); ++k)
+                    zs[k] = O::lds(&zb[((r + k) * 4 + f) * VB + NP * lane]);
+#pragma unroll
+                for (int w = 0; w < RW; ++w) {
+                    cen[f][w] = zs[R + w];
+                    if constexpr (APART) {
+                        V z = vmul(wz[0], zs[w + R - 2]);
+                        if (R == 3) z = vfma(wz[0], zs[w + R - 2], vmul(kz, vadd(zs[w], zs[w + 2 * R])));
+                        z = vfma(wz[1], zs[w + R - 1], z);
+                        z = vfma(wz[2], zs[w + R + 1], z);
+                        z = vfma(wz[3], zs[w + R + 2], z);
+                        y[f][w] = vfma(kc, cen[f][w], vadd(z, y[f][w]));
+                    }
+                }
+            }
         }
         V pin[4][RW];  // the pointwise input: U (S2, S3) or B (S4)
         if (CF::PU || CF::PA) {
