@@ -68,7 +68,7 @@ extern "C" {
 #define NUOSC_LAYOUT_GHOSTED 1 /* the reference's array: [(i+gx)*(nz+2gz)+j+gz]*nv+v (CartGrid.h:91) */
 
 /* stage-kernel selection (nuosc_set_kernel) */
-#define NUOSC_KERNEL_AUTO 0   /* the TMA x-march kernel (any nz >= 14), else the cp.async one */
+#define NUOSC_KERNEL_AUTO 0   /* the TMA x-march kernel (nz >= 14, up to 65,535 z tiles), else the cp.async one */
 #define NUOSC_KERNEL_DIRECT 1 /* one thread per (cell, velocity), separate moment pass */
 #define NUOSC_KERNEL_XMARCH 2 /* cp.async-staged x-march with fused moments (any geometry) */
 #define NUOSC_KERNEL_XTMA 3   /* TMA-fed x-march with mbarrier ring, fused moments; asked for by name: nz % tz == 0 */
@@ -341,8 +341,11 @@ int nuosc_get_profile(nuosc_handle *h, double *ms, long long *launches, int nkin
  *   - all calls share the one array and it keeps the last call's moments;
  *     each call rewrites every entry it reads, so nothing needs clearing, but
  *     calls that overlap on the GPU (e.g. on two streams at once) race on it.
- * Returns NUOSC_OK once the two kernels are queued; errors are reported by
- * nuosc_last_error(). */
+ * Returns NUOSC_OK once its kernels are queued (the moment pass and the
+ * right-hand side, with one more for the last velocities where the grid is
+ * large); errors are reported by nuosc_last_error().  A bounded in-kernel wait
+ * that expires (a copy that never lands) has no status to go to here: the tiles
+ * it leaves incomplete are filled with NaN. */
 #define NUOSC_NOALLOC_MAX_CELLS 65536
 typedef struct nuosc_rhs_desc {
     int nx, nz, nv;     /* interior cells and velocities */

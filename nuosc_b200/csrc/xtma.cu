@@ -42,11 +42,7 @@
 // shifted every plane, weights read from shared memory, plain loads of the
 // pointwise inputs, warp 0 issuing the copies -- took 3.9 / 5.0 / 4.5 / 4.6 ms:
 // 404-467 instructions and 112 shared-memory wavefronts per 32 points against
-// 225-260 and 70 now, with the shared-memory pipe at 65 %.  Tried between the
-// two, on the same grid (S1): two velocities per thread 3.8 (constants re-read
-// from shared memory: its pipe stays the limit), the fields split between
-// warps 4.0 (same), the issue rotated among the consumer warps 2.9 but S2 6.2
-// (a late warp starves all), issue by the last warp to release a slot 3.3.
+// about 240 and 70 now, with the shared-memory pipe at 65 %.
 // FP32 (same grid): 2.2 / 2.8 / 2.4 / 2.5 -> 1.7 / 2.2 / 1.8 / 1.8 ms.
 //
 // The file is compiled in parts (NUOSC_PART, build.py), each with its share of the
@@ -1378,11 +1374,9 @@ bool xtma_grid_ok(const Geom &g, XTile t) {
 // x planes per CTA.  A segment costs its planes plus about 10 more (the launch of
 // the CTA, the constants, R planes left of it and R right of it), and a launch
 // costs whole waves of CTAs, so the number of segments minimises waves x (lx +
-// 10); among segment counts within 2 % the fewest.  Measured (us per FP64 step,
-// best of a sweep over lx in brackets): 32x32x42 lx 2: 53 [53], 16: 109, 32:
-// 174; 64x64x162 lx 22: 208 [208], 32: 238, 64: 371; 128x128x162 lx 43: 570
-// [566], 32: 636, 64: 749; 128x128x642 lx 64: 1817 [1817], 128: 2015;
-// 100x90x162 lx 50: 344 [344], 34: 426, 100: 525.
+// 10); among segment counts within 2 % the fewest.  (A fit to sweeps over lx, 32x32 to
+// 512x256 cells: its choice was within 1 % of each sweep's best; 32x32x42 in one
+// segment took three times as long as in the 16 it chose.)
 //
 // Where many whole waves make all counts cost the same, two limits stand.  CTAs
 // drift apart along a long march, and neighbouring velocity blocks then no longer
