@@ -36,14 +36,14 @@
 //
 // What bounds it, measured on a 512 x 256 x 642 FP64 grid (KO6): S1 2.6 ms (2
 // state passes, 4.1 TB/s) is held by instruction latency at 8 consumer warps
-// per SM (two per scheduler: the partial sums alone take 96 registers); S2 4.5,
-// S3 3.1, S4 3.1 ms run at 4.8-5.2 TB/s of the 6.5 a plain copy reaches.  The
+// per SM (two per scheduler: the partial sums alone take 96 registers); S2 4.6,
+// S3 3.1, S4 3.1 ms run at 4.7-5.3 TB/s of the 6.5 a plain copy reaches.  The
 // form before -- 16 warps of one point per thread, a 7-deep register queue in x
 // shifted every plane, weights read from shared memory, plain loads of the
 // pointwise inputs, warp 0 issuing the copies -- took 3.9 / 5.0 / 4.5 / 4.6 ms:
 // 404-467 instructions and 112 shared-memory wavefronts per 32 points against
 // about 240 and 70 now, with the shared-memory pipe at 65 %.
-// FP32 (same grid): 2.2 / 2.8 / 2.4 / 2.5 -> 1.7 / 2.2 / 1.8 / 1.8 ms.
+// FP32 (same grid): 2.2 / 2.8 / 2.4 / 2.5 -> 1.7 / 2.2 / 1.7 / 1.8 ms.
 //
 // The file is compiled in parts (NUOSC_PART, build.py), each with its share of the
 // kernels: the whole in one piece takes 7 minutes.  (nvcc's --split-compile halves
@@ -52,7 +52,7 @@
 // written out: a loop for the fronts that complete no centre, loads in program
 // order, no branch on what is the same in every plane.  Against the better of the
 // two codes (geometric mean over 16 to 512 cells a side, 12 to 642 velocities):
-// steps FP64 1.04, FP32 1.11, calRHS 1.07 and 1.09, batches 1.01 to 1.13.
+// steps FP64 1.05, FP32 1.08, calRHS 1.07 and 1.09, batches 1.06 to 1.10.
 //
 // The march of one tile is a device function shared by two kernels: k_xtma
 // (one tile per CTA, one instance per launch) and k_xtma_batch (a persistent
@@ -1374,9 +1374,10 @@ bool xtma_grid_ok(const Geom &g, XTile t) {
 // x planes per CTA.  A segment costs its planes plus about 10 more (the launch of
 // the CTA, the constants, R planes left of it and R right of it), and a launch
 // costs whole waves of CTAs, so the number of segments minimises waves x (lx +
-// 10); among segment counts within 2 % the fewest.  (A fit to sweeps over lx, 32x32 to
-// 512x256 cells: its choice was within 1 % of each sweep's best; 32x32x42 in one
-// segment took three times as long as in the 16 it chose.)
+// 10); among segment counts within 2 % the fewest.  Measured (us per FP64 step, the choice in
+// brackets): 32x32x42 [2] 32, 4: 39, 16: 87, 32: 145; 64x64x162 [22] 138, 16: 196,
+// 32: 170, 64: 289; 128x128x162 [43] 483, 32: 522, 64: 608; 100x90x162 [50] 271,
+// 34: 351, 100: 468; 128x128x642 [64] 1825, 32: 1712, 128: 2037.
 //
 // Where many whole waves make all counts cost the same, two limits stand.  CTAs
 // drift apart along a long march, and neighbouring velocity blocks then no longer
@@ -1480,8 +1481,8 @@ cudaError_t launch_stage_xtma(const StageArgs<T> &a, int mode, bool ko6, XTile t
 
 // calRHS on the march: 2 state passes (plus the moment pass before it) instead
 // of the direct kernel's 13 or 9 loads per value from L2.  Whole call, moment
-// pass included: 128x128x642 FP64, KO6 1150 -> 567 us (140 of them the moment
-// pass); 250x130x162 FP32, KO4 296 -> 172 us.  The direct kernel stays for nz <
+// pass included: 128x128x642 FP64, KO6 1152 -> 474 us (140 of them the moment
+// pass); 250x130x162 FP32, KO4 301 -> 157 us.  The direct kernel stays for nz <
 // 14, for buffers without 16-byte rows and where rhs_xtma_pays says so.
 template <typename T>
 XTile rhs_tile(const Geom &g) {
